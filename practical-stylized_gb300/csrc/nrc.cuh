@@ -1,6 +1,8 @@
 // nrc.cuh -- neural radiance cache: shared definitions of the FP32 and BF16 (tcgen05) paths.
 #pragma once
 
+#include <cuda_bf16.h>
+
 #include "common.cuh"
 
 namespace sty {
@@ -54,6 +56,36 @@ constexpr int kNrcTcTrainMaxLayers = 6;
 uint32_t nrc_tc_train_ctas(uint32_t B);
 sty_status nrc_tc_train(const NrcNet &n, const uint16_t *w_img, uint32_t B, const float *input, const float *target,
                         float *part, size_t np, float *loss, uint32_t ctas, cudaStream_t st);
+
+// FP32 network on the tensor cores (nrc_f32tc.cu): the hidden layers' weights as three BF16 pieces,
+// per layer three K-major operand images of 64 x 64. The pieces sum to w (1 + kNrcUnbias): tcgen05
+// truncates its accumulations, which takes ~0.7 x 2^-24 off a layer's outputs on average, and the
+// third piece, whose last place is 2^-25 of w, gives it back:
+// without it the outputs of a 5 x 64 network were 2.0e-7 too small on average, with it 1e-8 too large,
+// and |mean| <= 3e-8 over 1 to 8 layers.
+constexpr float kNrcUnbias = 4.2e-8f;
+size_t nrc_f32tc_image_elems(const NrcNet &n);
+// piece images of hidden weight i (flat parameter index, < layers * 64 * 64) for the value v
+__device__ __forceinline__ void nrc_store_pieces(uint16_t *img, size_t i, float v) {
+    const uint32_t e = (uint32_t)(i & (kNrcWidth * kNrcWidth - 1)), row = e / kNrcWidth, k = e % kNrcWidth;
+    uint16_t *dst = img + (i - e) * 3 + ((row >> 3) * 8u + (k >> 3)) * 64u + (row & 7u) * 8u + (k & 7u);
+    float r = v;
+#pragma unroll
+    for (int p = 0; p < 3; p++) {
+        const __nv_bfloat16 b = __float2bfloat16_rn(r);
+        dst[p * kNrcWidth * kNrcWidth] = __bfloat16_as_ushort(b);
+        r -= __bfloat162float(b);
+        if (p == 1) r = fmaf(v, kNrcUnbias, r);
+    }
+}
+sty_status nrc_f32tc_pack(const NrcNet &n, const float *w, uint16_t *img, cudaStream_t st);
+sty_status nrc_f32tc_forward(const NrcNet &n, const float *w, const uint16_t *img, uint64_t count, const float *input,
+                             float *output, cudaStream_t st);
+// forward, relative-L2 gradient and backward of a batch: the activations (row 0 the encoding) and the
+// pre-activation gradients (row `layers` the loss gradient) to acts / dpre [layers + 1][B][64], the
+// loss added to *loss
+sty_status nrc_f32tc_train(const NrcNet &n, const float *w, const uint16_t *img, uint32_t B, const float *input,
+                           const float *target, float *acts, float *dpre, float *loss, cudaStream_t st);
 
 // The reference's composite-encoding network (nrc_grid.cu)
 struct GridModel;

@@ -104,6 +104,19 @@ __device__ __forceinline__ uint32_t pack2_relu_bf16(float lo, float hi) {  // ma
     asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
     return r;
 }
+// A value that is the same in the whole warp, as one the compiler knows to be: operands of MMAs that
+// come from it stay in uniform registers. MMAs are issued by one elected lane of a warp that enters
+// the branch as a whole, with uniform operands: an MMA of M = 128, K = 16 with A in TMEM then takes 32
+// cycles at N = 64 and 9 at N = 16 (the tensor pipe's rate), where `if (threadIdx.x == 0)`, which moves
+// every operand from vector registers, takes 45 in a tight loop and 100 or more between other code
+// (1000 MMAs from one warp, clock64 to the commit). With A in shared memory N = 64 takes 48: its 6 KB
+// of operands at 128 B per cycle.
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 // named barrier over n threads (id 0 is __syncthreads), and its AND-reduction form
 __device__ __forceinline__ void bar_sync_n(uint32_t id, uint32_t n) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
