@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "fastmod.h"
 
 namespace sty {
 
@@ -44,6 +45,71 @@ __device__ __forceinline__ void nrc_encode(const NrcNet &n, const float *x, floa
     for (; o < kNrcWidth; o++) enc[o] = 0.0f;
 }
 
+// The frequency table of the neural-cache workload network (11 inputs, octaves 4,4,4,3,3,3,3,2,2,2,2 -> 64
+// columns) fixed at compile time: columns 32 HALF .. 32 HALF + 31 of nrc_encode, every column in a static
+// register, no per-pair branch or table lookup. x holds the inputs the half needs: 0 .. 4, or 4 .. 10 (input
+// 4's octaves lie in both halves).
+constexpr int kNrcC4Half = 7;
+constexpr int kNrcC4Dims = 11;
+__device__ constexpr int kNrcC4Freqs[kNrcC4Dims] = {4, 4, 4, 3, 3, 3, 3, 2, 2, 2, 2};
+inline bool nrc_is_c4(const NrcNet &n) {
+    const int f[kNrcC4Dims] = {4, 4, 4, 3, 3, 3, 3, 2, 2, 2, 2};
+    if (n.in_dims != kNrcC4Dims) return false;
+    for (int d = 0; d < kNrcC4Dims; d++)
+        if ((int)n.freqs[d] != f[d]) return false;
+    return true;
+}
+template <int HALF>
+__device__ __forceinline__ void nrc_encode_c4(const float (&x)[kNrcC4Half], float (&enc)[32]) {
+    int o = 0;  // pairs before dim d
+#pragma unroll
+    for (int d = 0; d < kNrcC4Dims; d++) {
+        if (o < 16 * HALF + 16 && o + kNrcC4Freqs[d] > 16 * HALF) {
+            float s, c;
+            sincospif(x[d - 4 * HALF], &s, &c);
+#pragma unroll
+            for (int k = 0; k < kNrcC4Freqs[d]; k++) {
+                const int p = o + k - 16 * HALF;
+                if (p >= 0 && p < 16) {
+                    enc[2 * p] = s;
+                    enc[2 * p + 1] = c;
+                }
+                const float s2 = 2.0f * s * c;
+                c = fmaf(-2.0f * s, s, 1.0f);
+                s = s2;
+            }
+        }
+        o += kNrcC4Freqs[d];
+    }
+}
+
+// The rows of a training batch: sample b is row `index(b)` of input / target. A sampled batch draws its rows
+// uniformly from `count` (collect_batch, akari_tcnn.cu:15-38: one Pcg32 stream per sample of the run, number
+// base + b); an explicit one takes them in order. The training kernels gather by it themselves: the copy of
+// the batch it replaces was a launch and 5 to 8 us.
+__device__ __forceinline__ uint32_t nrc_pcg_step(uint64_t &state, uint64_t inc) {
+    const uint64_t old = state;
+    state = old * 0x5851f42d4c957f2dULL + inc;
+    const uint32_t xs = (uint32_t)(((old >> 18) ^ old) >> 27);
+    const uint32_t rot = (uint32_t)(old >> 59);
+    return (xs >> rot) | (xs << ((~rot + 1u) & 31u));
+}
+struct NrcRows {
+    const float *input, *target;
+    bool sampled;
+    uint64_t seed, base, count, magic;  // magic = fastmod_magic(count): r % count without a 64-bit division
+    __device__ __forceinline__ uint64_t index(uint32_t b) const {
+        if (!sampled) return b;
+        uint64_t st = 0;
+        const uint64_t inc = ((base + b) << 1) | 1ull;
+        nrc_pcg_step(st, inc);
+        st += seed;
+        nrc_pcg_step(st, inc);
+        const uint64_t hi = nrc_pcg_step(st, inc);
+        return fastmod((hi << 32) | nrc_pcg_step(st, inc), count, magic);
+    }
+};
+
 // BF16 tensor-core path (nrc_tc.cu)
 struct NrcTcWeights;  // device buffers in the UMMA shared-memory image layout
 sty_status nrc_tc_pack(const NrcNet &n, const float *w_fp32, uint16_t *w_img, cudaStream_t st);
@@ -54,10 +120,17 @@ sty_status nrc_tc_forward(const NrcNet &n, const uint16_t *w_img, uint64_t count
 // of B samples on `ctas` CTAs (nrc_tc_train_ctas); per-CTA gradient sums go to part[ctas][np].
 constexpr int kNrcTcTrainMaxLayers = 6;
 uint32_t nrc_tc_train_ctas(uint32_t B);
-sty_status nrc_tc_train(const NrcNet &n, const uint16_t *w_img, uint32_t B, const float *input, const float *target,
-                        float *part, size_t np, float *loss, uint32_t ctas, cudaStream_t st);
+sty_status nrc_tc_train(const NrcNet &n, const uint16_t *w_img, uint32_t B, const NrcRows &rows, float *part, size_t np, float *loss, uint32_t ctas, cudaStream_t st);
 
-// FP32 network on the tensor cores (nrc_f32tc.cu): the hidden layers' weights as three BF16 pieces,
+// BF16 operand image (nrc_tc_pack) of parameter i for the value v: per layer a K-major image, the output
+// layer's behind the hidden ones
+__device__ __forceinline__ void nrc_store_bf16(uint16_t *img, size_t i, float v) {
+    const uint32_t e = (uint32_t)(i & (kNrcWidth * kNrcWidth - 1)), row = e / kNrcWidth, k = e % kNrcWidth;
+    img[(i - e) + ((row >> 3) * 8u + (k >> 3)) * 64u + (row & 7u) * 8u + (k & 7u)] =
+        __bfloat16_as_ushort(__float2bfloat16_rn(v));
+}
+
+// FP32 inference on the tensor cores (nrc_f32tc.cu): the hidden layers' weights as three BF16 pieces,
 // per layer three K-major operand images of 64 x 64. The pieces sum to w (1 + kNrcUnbias): tcgen05
 // truncates its accumulations, which takes ~0.7 x 2^-24 off a layer's outputs on average, and the
 // third piece, whose last place is 2^-25 of w, gives it back:
@@ -81,12 +154,6 @@ __device__ __forceinline__ void nrc_store_pieces(uint16_t *img, size_t i, float 
 sty_status nrc_f32tc_pack(const NrcNet &n, const float *w, uint16_t *img, cudaStream_t st);
 sty_status nrc_f32tc_forward(const NrcNet &n, const float *w, const uint16_t *img, uint64_t count, const float *input,
                              float *output, cudaStream_t st);
-// forward, relative-L2 gradient and backward of a batch: the activations (row 0 the encoding) and the
-// pre-activation gradients (row `layers` the loss gradient) to acts / dpre [layers + 1][B][64], the
-// loss added to *loss
-sty_status nrc_f32tc_train(const NrcNet &n, const float *w, const uint16_t *img, uint32_t B, const float *input,
-                           const float *target, float *acts, float *dpre, float *loss, cudaStream_t st);
-
 // The reference's composite-encoding network (nrc_grid.cu)
 struct GridModel;
 sty_status grid_create(const sty_nrc_grid_config *c, GridModel **out, size_t *n_params, size_t *n_mlp);

@@ -10,13 +10,12 @@
 // the bias of the cuts given back, nrc.cuh; 4.1e-7 with FMA chains on the CUDA cores).
 //
 // Bound: the epilogues' instructions (load, ReLU, split, store of every activation): with 4 of the 18 MMAs
-// of a layer the kernel takes 95 % of its time. 2 073 600 queries 0.37 ms, 129 601 queries 31 us (the
-// register-tiled CUDA-core kernel this replaces: 1.99 ms, 164 us); forward + backward of 2^14 samples
-// 27 us (109 us).
+// of a layer the kernel takes 95 % of its time. 2 073 600 queries 0.33 ms, 129 601 queries 29 us (the
+// register-tiled CUDA-core kernel this replaces: 1.99 ms, 164 us).
 //
-// k_nrc_f32tc<false>: inference. k_nrc_f32tc<true>: the training step's forward, loss gradient and
-// backward in one kernel (the activations and pre-activation gradients go to global memory in FP32
-// for the weight-gradient kernel, nrc.cu).
+// Inference only: the training step stays on the CUDA cores (nrc.cu). Adam divides by the root of the
+// squared gradient, so weights whose gradient is all rounding follow that rounding; a training run
+// with other sums agrees with the earlier one only until such a weight matters.
 // Two tiles of 128 samples per CTA, one CTA per SM, so one tile's epilogue runs under the other's
 // MMAs. A tile has 8 warps: a sample is a TMEM lane and two threads, 32 of the 64 units each (with one
 // thread per sample the SM held 8 warps, and the encoder and the splits waited on their own latency:
@@ -24,9 +23,9 @@
 // 0.54 with two threads). TMEM per tile: two 64-column accumulators (D1, D2: a layer's output is their sum),
 // the next layer's A operand, 3 pieces of 32 columns, and 32 columns for the output layer's exchange.
 // Weights: per layer three K-major images of 64 x 64 in shared memory, w1 and w2 adjacent, so one
-// N = 128 MMA takes a piece of the activations to both. The backward reads the same images MN-major.
-// The 64 -> <= 16 output layer and its transpose stay on the CUDA cores: an MMA round trip costs more
-// than its 192 FMAs a sample.
+// N = 128 MMA takes a piece of the activations to both.
+// The 64 -> <= 16 output layer stays on the CUDA cores: an MMA round trip costs more than its 192 FMAs a
+// sample.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -60,11 +59,7 @@ struct Args {
     const float *wout;  // FP32 output layer
     uint64_t count;
     const float *input;
-    float *output;        // inference: predictions; training: unused
-    const float *target;  // training
-    float *acts;          // [layers + 1][count][64]
-    float *dpre;          // [layers + 1][count][64]
-    float *loss;
+    float *output;
     uint32_t *status;
 };
 
@@ -101,12 +96,6 @@ __device__ __forceinline__ void store_a(uint32_t areg, const float (&h)[32]) {
 #pragma unroll
     for (int p = 0; p < 3; p++) tmem_st16(areg + 32u * p, q[p]);
 }
-__device__ __forceinline__ void store_row(float *dst, const float (&h)[32]) {
-#pragma unroll
-    for (int k = 0; k < 32; k += 4)
-        *reinterpret_cast<float4 *>(dst + k) = make_float4(h[k], h[k + 1], h[k + 2], h[k + 3]);
-}
-
 // The six piece products of a layer, 4 K steps each, small ones first.
 __device__ __forceinline__ void issue_forward(uint32_t d, uint32_t a, uint32_t w) {
     const uint32_t wide = idesc_bf16(TM, 2 * W), one = idesc_bf16(TM, W);
@@ -123,58 +112,6 @@ __device__ __forceinline__ void issue_forward(uint32_t d, uint32_t a, uint32_t w
 #pragma unroll
     for (int kk = 2; kk < 4; kk++) mma_ts(d + 64u, a + 8u * kk, make_desc(w + 256u * kk), one, 1u);
 }
-// dH = dP W: the image read MN-major (its rows are the summed index), 6 x 4 MMAs of N = 64
-__device__ __forceinline__ void issue_backward(uint32_t d, uint32_t a, uint32_t w) {
-    const uint32_t id = idesc_bf16(TM, W, 0, 1);
-    auto prod = [&](uint32_t acc_col, uint32_t pa, uint32_t pw, int k0, int k1, bool fresh) {
-#pragma unroll
-        for (int kk = k0; kk < k1; kk++)
-            mma_ts(d + acc_col, a + 32u * pa + 8u * kk, make_desc_mn(w + pw * kImg + 2048u * kk), id,
-                   (fresh && kk == k0) ? 0u : 1u);
-    };
-    prod(64u, 1, 1, 0, 4, true);
-    prod(64u, 2, 0, 0, 4, false);
-    prod(64u, 0, 2, 0, 4, false);
-    prod(64u, 0, 1, 0, 4, false);
-    prod(0u, 1, 0, 0, 4, true);
-    prod(64u, 0, 0, 2, 4, false);
-    prod(0u, 0, 0, 0, 2, false);
-}
-
-constexpr int kC4Dims = 11;
-__device__ constexpr int kC4Freqs[kC4Dims] = {4, 4, 4, 3, 3, 3, 3, 2, 2, 2, 2};
-bool is_c4(const NrcNet &n) {
-    if (n.in_dims != kC4Dims) return false;
-    const int f[kC4Dims] = {4, 4, 4, 3, 3, 3, 3, 2, 2, 2, 2};
-    for (int d = 0; d < kC4Dims; d++)
-        if ((int)n.freqs[d] != f[d]) return false;
-    return true;
-}
-// columns 32 HALF .. 32 HALF + 31 of the encoding with the workload's frequency table, every column in a
-// static register; the arithmetic of nrc_encode
-template <int HALF>
-__device__ __forceinline__ void encode_c4(const float *x, float (&enc)[32]) {
-    int o = 0;  // pairs before dim d
-#pragma unroll
-    for (int d = 0; d < kC4Dims; d++) {
-        if (o < 16 * HALF + 16 && o + kC4Freqs[d] > 16 * HALF) {
-            float s, c;
-            sincospif(x[d], &s, &c);
-#pragma unroll
-            for (int k = 0; k < kC4Freqs[d]; k++) {
-                const int p = o + k - 16 * HALF;
-                if (p >= 0 && p < 16) {
-                    enc[2 * p] = s;
-                    enc[2 * p + 1] = c;
-                }
-                const float s2 = 2.0f * s * c;
-                c = fmaf(-2.0f * s, s, 1.0f);
-                s = s2;
-            }
-        }
-        o += kC4Freqs[d];
-    }
-}
 __device__ __forceinline__ void tmem_st4(uint32_t taddr, const float (&v)[4]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "f"(v[0]), "f"(v[1]), "f"(v[2]),
                  "f"(v[3])
@@ -187,7 +124,7 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
 }
 
 // OM: output columns kept in registers (4, or 16 for wider outputs)
-template <bool TRAIN, int OM>
+template <int OM>
 __global__ void __launch_bounds__(kGT * kTiles, 1) k_nrc_f32tc(const Args a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar[kTiles], wbar;
@@ -197,8 +134,6 @@ __global__ void __launch_bounds__(kGT * kTiles, 1) k_nrc_f32tc(const Args a) {
     const bool issuer = warp % (kGT / 32) == 0;  // the tile's issuing warp
     const uint32_t bar_id = 1u + (uint32_t)grp;
     const int L = a.n.layers, O = a.n.out_dims;
-    // TRAIN: which units of each layer were positive, a word per layer and thread
-    uint32_t *mask = reinterpret_cast<uint32_t *>(smem + (size_t)L * kLayer) + tid;
     for (int e = tid; e < O * W; e += kGT * kTiles) wo[e] = a.wout[e];
     if (tid == 0) {
         for (int g = 0; g < kTiles; g++)
@@ -228,27 +163,26 @@ __global__ void __launch_bounds__(kGT * kTiles, 1) k_nrc_f32tc(const Args a) {
     const uint32_t lane_off = ((uint32_t)(warp & 3) * 32u) << 16;
     const uint32_t mine = tmem + lane_off + 32u * half;                 // this thread's columns of D1 (D2: + 64)
     const uint32_t amine = areg + lane_off + 16u * half;                // of the A pieces
-    const uint32_t exch = tmem + lane_off + 224u;                       // the output layer's halves, 16 columns each
+    const uint32_t exch = tmem + lane_off + 224u;                       // the upper half's share of the output layer, columns 16 .. 31
     const float *wo_mine = wo + 32 * half;
     const uint32_t wbase = smem_u32(smem);
     uint64_t *bar = &mbar[grp];
     uint32_t phase = 0;
     bool failed = false;  // uniform over the tile's threads
-    float lsum = 0.0f;
-    const float norm = 1.0f / ((float)a.count * (float)O);
 
-    auto wait_mma = [&]() -> bool {
-        const bool got = mbar_wait(bar, phase, a.status);
+    bool ok = true;  // this thread's waits came through; the tile's threads agree on it in publish()
+    auto wait_mma = [&]() {
+        ok = mbar_wait(bar, phase, a.status) && ok;
         phase ^= 1u;
-        if (!bar_and_n(bar_id, kGT, got)) return false;
         fence_after();
-        return true;
     };
-    auto publish = [&]() {  // the tile's TMEM accesses so far come before those issued next
+    // the tile's TMEM accesses so far come before those issued next; false if any wait ran out
+    auto publish = [&]() -> bool {
         tmem_wait_st();
         fence_before();
-        bar_sync_n(bar_id, kGT);
+        const bool all = bar_and_n(bar_id, kGT, ok);
         fence_after();
+        return all;
     };
     auto load_sum = [&](float (&h)[32]) {
         float u[32];
@@ -265,6 +199,20 @@ __global__ void __launch_bounds__(kGT * kTiles, 1) k_nrc_f32tc(const Args a) {
 
     bool loaded = false;  // the weight images have arrived
     const uint64_t ntiles = (a.count + TM - 1) / TM;
+    // the workload encoder's inputs of this thread's half, loaded a tile ahead (asm volatile: not sunk to
+    // their use)
+    float xr[kNrcC4Half];
+    auto load_x = [&](uint64_t tl) {
+        const uint64_t r = tl * TM + t;
+        const bool v = a.c4 && tl < ntiles && r < a.count;
+        const float *p = a.input + r * kNrcC4Dims + 4 * half;
+#pragma unroll
+        for (int i = 0; i < kNrcC4Half; i++) {
+            xr[i] = 0.0f;
+            if (v && (half == 1 || i < 5)) asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(xr[i]) : "l"(p + i));
+        }
+    };
+    load_x(blockIdx.x + (uint64_t)gridDim.x * grp);
     // one tile per SM before any SM gets a second
     for (uint64_t tile = blockIdx.x + (uint64_t)gridDim.x * grp; tile < ntiles && !failed;
          tile += (uint64_t)gridDim.x * kTiles) {
@@ -276,26 +224,25 @@ __global__ void __launch_bounds__(kGT * kTiles, 1) k_nrc_f32tc(const Args a) {
             for (int k = 0; k < 32; k++) h[k] = 0.0f;
         } else if (a.c4) {
             if (half == 0)
-                encode_c4<0>(a.input + row * kC4Dims, h);
+                nrc_encode_c4<0>(xr, h);
             else
-                encode_c4<1>(a.input + row * kC4Dims, h);
+                nrc_encode_c4<1>(xr, h);
         } else {
             float enc[W];
             nrc_encode(a.n, a.input + row * a.n.in_dims, enc);
 #pragma unroll
             for (int k = 0; k < 32; k++) h[k] = half == 0 ? enc[k] : enc[32 + k];
         }
-        if (TRAIN && valid) store_row(a.acts + row * W + 32 * half, h);
+        load_x(tile + (uint64_t)gridDim.x * kTiles);
         store_a(amine, h);
         if (!loaded) {
-            const bool got = mbar_wait(&wbar, 0, a.status);
-            if (!bar_and_n(bar_id, kGT, got)) {
-                failed = true;
-                break;
-            }
+            ok = mbar_wait(&wbar, 0, a.status);
             loaded = true;
         }
-        publish();
+        if (!publish()) {
+            failed = true;
+            break;
+        }
         float pred[OM];
 #pragma unroll
         for (int c = 0; c < OM; c++) pred[c] = 0.0f;
@@ -304,21 +251,10 @@ __global__ void __launch_bounds__(kGT * kTiles, 1) k_nrc_f32tc(const Args a) {
                 issue_forward(tmem, areg, wbase + (uint32_t)l * kLayer);
                 mma_commit(bar);
             }
-            if (!wait_mma()) {
-                failed = true;
-                break;
-            }
+            wait_mma();
             load_sum(h);
-            uint32_t pos = 0;
 #pragma unroll
-            for (int k = 0; k < 32; k++) {
-                h[k] = fmaxf(h[k], 0.0f);
-                if (TRAIN) pos |= (h[k] > 0.0f ? 1u : 0u) << k;
-            }
-            if (TRAIN) {
-                mask[l * (kGT * kTiles)] = pos;
-                if (valid) store_row(a.acts + ((size_t)(l + 1) * a.count + row) * W + 32 * half, h);
-            }
+            for (int k = 0; k < 32; k++) h[k] = fmaxf(h[k], 0.0f);
             if (l + 1 < L) {
                 store_a(amine, h);
             } else {  // output layer: this thread's 32 units, then the two halves' sums
@@ -337,97 +273,39 @@ __global__ void __launch_bounds__(kGT * kTiles, 1) k_nrc_f32tc(const Args a) {
 #pragma unroll
                 for (int c = 0; c < OM; c += 4) {
                     const float v[4] = {pred[c], pred[c + 1], pred[c + 2], pred[c + 3]};
-                    tmem_st4(exch + 16u * half + c, v);
+                    if (half == 1) tmem_st4(exch + 16u + c, v);
                 }
             }
-            publish();
+            if (!publish()) {
+                failed = true;
+                break;
+            }
         }
         if (failed) break;
-        if (TRAIN || half == 0) {
+        // (the next tile's first publish orders these reads before the exchange is written again)
+        if (half == 0) {
 #pragma unroll
             for (int c = 0; c < OM; c += 4) {
                 float v[4];
-                tmem_ld4(exch + 16u * (half ^ 1) + c, v);
+                tmem_ld4(exch + 16u + c, v);
                 tmem_wait_ld();
 #pragma unroll
-                for (int e = 0; e < 4; e++) pred[c + e] += v[e];
-            }
-        }
-        if constexpr (!TRAIN) {
-            // (the next tile's first publish orders this read before the exchange is written again)
-            if (valid && half == 0)
-#pragma unroll
-                for (int c = 0; c < OM; c++)
-                    if (c < O) a.output[row * O + c] = pred[c];
-        } else {
-            // ---- relative L2 (prediction constant in the denominator), then dH_{L-1} = W_out^T g
-            float g[OM];
-#pragma unroll
-            for (int c = 0; c < OM; c++) {
-                g[c] = 0.0f;
-                if (c < O && valid) {
-                    const float p = pred[c], tg = a.target[row * O + c];
-                    const float den = p * p + 0.01f;
-                    g[c] = 2.0f * (p - tg) / den * norm;
-                    if (half == 0) {
-                        lsum += (p - tg) * (p - tg) / den;
-                        a.dpre[((size_t)L * a.count + row) * W + c] = g[c];
-                    }
-                }
-            }
-            for (int l = L - 1; l >= 0; l--) {
-                if (l == L - 1) {
-#pragma unroll
-                    for (int k = 0; k < 32; k++) h[k] = 0.0f;
-#pragma unroll
-                    for (int c = 0; c < OM; c++)
-                        if (c < O) {
-#pragma unroll
-                            for (int k = 0; k < 32; k += 4) {
-                                const float4 w4 = *reinterpret_cast<const float4 *>(wo_mine + c * W + k);
-                                h[k] = fmaf(w4.x, g[c], h[k]);
-                                h[k + 1] = fmaf(w4.y, g[c], h[k + 1]);
-                                h[k + 2] = fmaf(w4.z, g[c], h[k + 2]);
-                                h[k + 3] = fmaf(w4.w, g[c], h[k + 3]);
-                            }
-                        }
-                } else {
-                    load_sum(h);
-                }
-                const uint32_t pos = mask[l * (kGT * kTiles)];
-#pragma unroll
-                for (int k = 0; k < 32; k++) h[k] = (pos >> k) & 1u ? h[k] : 0.0f;
-                if (valid) store_row(a.dpre + ((size_t)l * a.count + row) * W + 32 * half, h);
-                if (l > 0) store_a(amine, h);
-                publish();
-                if (l == 0) break;
-                if (issuer && elect_one()) {
-                    issue_backward(tmem, areg, wbase + (uint32_t)l * kLayer);
-                    mma_commit(bar);
-                }
-                if (!wait_mma()) {
-                    failed = true;
-                    break;
-                }
+                for (int e = 0; e < 4; e++)
+                    if (valid && c + e < O) a.output[row * O + c + e] = pred[c + e] + v[e];
             }
         }
     }
     if (failed) mbar_wait(bar, phase, a.status);  // one more bounded wait before the columns are released
     if (!loaded) mbar_wait(&wbar, 0, a.status);   // no copy in flight when the block ends
-    if (TRAIN) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-        if ((tid & 31) == 0 && a.loss && lsum != 0.0f) atomicAdd(a.loss, lsum * norm);
-    }
     fence_before();
     __syncthreads();
     fence_after();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_slot) : "memory");
 }
 
-template <bool TRAIN, int OM>
+template <int OM>
 sty_status launch(Args a, cudaStream_t st) {
-    a.c4 = is_c4(a.n) ? 1 : 0;
+    a.c4 = nrc_is_c4(a.n) ? 1 : 0;
     a.status = device_status_ptr();
     if (!a.status) {
         set_error("device status word unavailable");
@@ -437,12 +315,11 @@ sty_status launch(Args a, cudaStream_t st) {
     STY_TRY(check_cuda(cudaGetDevice(&dev), "cudaGetDevice"));
     STY_TRY(check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr SMs"));
     // at least 120 KB so that one CTA (and its 512 TMEM columns) owns the SM
-    const size_t need = (size_t)a.n.layers * (kLayer + (TRAIN ? kGT * kTiles * 4 : 0));
-    const size_t smem = std::max<size_t>(need, 122880);
-    STY_TRY(check_cuda(cudaFuncSetAttribute(k_nrc_f32tc<TRAIN, OM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    const size_t smem = std::max<size_t>((size_t)a.n.layers * kLayer, 122880);
+    STY_TRY(check_cuda(cudaFuncSetAttribute(k_nrc_f32tc<OM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                        "attr k_nrc_f32tc"));
     const uint64_t ntiles = (a.count + TM - 1) / TM;
-    k_nrc_f32tc<TRAIN, OM><<<(unsigned)std::min<uint64_t>(ntiles, (uint64_t)sms), kGT * kTiles, smem, st>>>(a);
+    k_nrc_f32tc<OM><<<(unsigned)std::min<uint64_t>(ntiles, (uint64_t)sms), kGT * kTiles, smem, st>>>(a);
     return check_launch("k_nrc_f32tc");
 }
 
@@ -463,21 +340,7 @@ sty_status nrc_f32tc_forward(const NrcNet &n, const float *w, const uint16_t *im
     a.count = count;
     a.input = input;
     a.output = output;
-    return n.out_dims <= 4 ? launch<false, 4>(a, st) : launch<false, kNrcOutPad>(a, st);
-}
-sty_status nrc_f32tc_train(const NrcNet &n, const float *w, const uint16_t *img, uint32_t B, const float *input,
-                           const float *target, float *acts, float *dpre, float *loss, cudaStream_t st) {
-    Args a{};
-    a.n = n;
-    a.img = img;
-    a.wout = w + nrc_w_offset(n.layers);
-    a.count = B;
-    a.input = input;
-    a.target = target;
-    a.acts = acts;
-    a.dpre = dpre;
-    a.loss = loss;
-    return n.out_dims <= 4 ? launch<true, 4>(a, st) : launch<true, kNrcOutPad>(a, st);
+    return n.out_dims <= 4 ? launch<4>(a, st) : launch<kNrcOutPad>(a, st);
 }
 
 }  // namespace sty

@@ -75,27 +75,15 @@ __device__ __forceinline__ void encode_row_pack(const EncPlan &e, const float *x
     }
 }
 
-// The same encoding with the frequency table of the neural-cache workload network (11 inputs,
-// octaves 4,4,4,3,3,3,3,2,2,2,2 -> 64 columns) fixed at compile time: every pair lands in a static
-// register, no per-pair branch or table lookup.
-constexpr int kC4Dims = 11;
-__device__ constexpr int kC4Freqs[kC4Dims] = {4, 4, 4, 3, 3, 3, 3, 2, 2, 2, 2};
-bool is_c4(const NrcNet &n) {
-    if (n.in_dims != kC4Dims) return false;
-    const int f[kC4Dims] = {4, 4, 4, 3, 3, 3, 3, 2, 2, 2, 2};
-    for (int d = 0; d < kC4Dims; d++)
-        if ((int)n.freqs[d] != f[d]) return false;
-    return true;
-}
 // the packed BF16 encoding of an input row held in registers (has = false: a padding row of zeros)
-__device__ __forceinline__ void encode_c4_pack(const float (&xin)[kC4Dims], bool has, uint32_t (&q)[kNrcWidth / 2]) {
+__device__ __forceinline__ void encode_c4_pack(const float (&xin)[kNrcC4Dims], bool has, uint32_t (&q)[kNrcWidth / 2]) {
     int o = 0;
 #pragma unroll
-    for (int d = 0; d < kC4Dims; d++) {
+    for (int d = 0; d < kNrcC4Dims; d++) {
         float s, c;
         sincospif(xin[d], &s, &c);
 #pragma unroll
-        for (int k = 0; k < kC4Freqs[d]; k++) {
+        for (int k = 0; k < kNrcC4Freqs[d]; k++) {
             q[o++] = has ? pack2_bf16(s, c) : 0u;
             const float s2 = 2.0f * s * c;
             c = fmaf(-2.0f * s, s, 1.0f);
@@ -111,9 +99,9 @@ __device__ __forceinline__ void store_row(const uint32_t (&q)[kNrcWidth / 2], ui
 }
 __device__ __forceinline__ void encode_any_pack(const EncPlan &e, bool c4, const float *x, uint32_t (&q)[kNrcWidth / 2]) {
     if (c4) {
-        float xin[kC4Dims];
+        float xin[kNrcC4Dims];
 #pragma unroll
-        for (int d = 0; d < kC4Dims; d++) xin[d] = x ? x[d] : 0.0f;
+        for (int d = 0; d < kNrcC4Dims; d++) xin[d] = x ? x[d] : 0.0f;
         encode_c4_pack(xin, x != nullptr, q);
     } else {
         encode_row_pack(e, x, q);
@@ -133,6 +121,14 @@ __device__ __forceinline__ void encode_row(const EncPlan &e, const float *x, uin
 }
 
 
+// a global load issued where it is written (an asm volatile is not moved past the other volatile
+// asm of the step loop), so its latency overlaps the steps before the value's first use
+__device__ __forceinline__ float ld_early(const float *p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
 struct TcArgs {
     NrcNet n;
     EncPlan plan;
@@ -149,11 +145,14 @@ struct TcArgs {
 // accumulator and the next layer's A operand, 32 columns of BF16 pairs: element k of row m in lane
 // m, column k / 2, half k % 2), an mbarrier and a named barrier. The activations never touch shared
 // memory: per layer the warpgroup tcgen05.ld's its accumulator rows, applies ReLU and BF16 rounding
-// and tcgen05.st's the row as the next layer's A; thread 0 issues 4 x tcgen05.mma (A from TMEM at
-// +8 columns per K = 16 step, B the layer's weight image; N = 64, or 16 for the output layer) and
-// commits to the mbarrier. Shared memory then carries only the B operands (2 KB per MMA instead of
-// 6 KB plus a 16 KB activation store per layer); 5 tiles are in flight per SM (5 x 96 of the 512
-// TMEM columns).
+// and tcgen05.st's the row as the next layer's A; an elected lane of its first warp issues
+// 4 x tcgen05.mma (A from TMEM at +8 columns per K = 16 step, B the layer's weight image; N = 64, or
+// 16 for the output layer) and commits to the mbarrier. 5 tiles are in flight per SM (5 x 96 of the
+// 512 TMEM columns); each tile's input row is loaded a tile ahead.
+// Bound: instruction issue (~1000 per warp and tile, 11 sincospif among them: 57 us of 2 073 600 queries at
+// one per cycle) with 5 warps a scheduler. 2 073 600 queries: 129 us before, 111 with MMAs issued from
+// a uniform warp, one barrier a layer instead of two and weights that arrive under the first encoding,
+// 93 with the input row a tile ahead. Two threads per sample (4 tiles, 32 warps) measured 126.
 constexpr int kFwdWG = 5;
 constexpr uint32_t kFwdCols = 96;
 __device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
@@ -177,53 +176,77 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&q)[32
 }
 __global__ void __launch_bounds__(128 * kFwdWG, 1) k_nrc_fwd_tc(const TcArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t mbar[kFwdWG];
+    __shared__ uint64_t mbar[kFwdWG], wbar;
     __shared__ uint32_t tmem_slot;
-    const int tid = threadIdx.x, warp = tid >> 5, wg = tid >> 7, t = tid & 127;
+    const int tid = threadIdx.x, warp = (int)uniform(threadIdx.x >> 5), wg = warp >> 2, t = tid & 127;
     const uint32_t bar_id = 1u + (uint32_t)wg;
     const int L = a.n.layers;
     const uint32_t wbytes = (uint32_t)(L * W * W + kNrcOutPad * W) * 2u;
-    uint8_t *wimg = smem;
 
-    for (uint32_t o = tid * 16u; o < wbytes; o += 128u * kFwdWG * 16u)
-        *reinterpret_cast<uint4 *>(wimg + o) =
-            *reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(a.wimg) + o);
     if (tid == 0) {
         for (int g = 0; g < kFwdWG; g++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[g])) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&wbar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        // the weight images, copied while the first tiles are encoded
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&wbar)), "r"(wbytes) : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         smem_u32(smem)),
+                     "l"(a.wimg), "r"(wbytes), "r"(smem_u32(&wbar))
+                     : "memory");
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    fence_async_smem();
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = tmem_slot + kFwdCols * (uint32_t)wg;  // accumulator
-    const uint32_t areg = tmem + 64u;                            // A operand of the next layer
+    const uint32_t tmem = uniform(tmem_slot) + kFwdCols * (uint32_t)wg;  // accumulator
+    const uint32_t areg = tmem + 64u;                                     // A operand of the next layer
     const uint32_t lane_off = ((uint32_t)(warp & 3) * 32u) << 16;
-    const uint32_t wbase = smem_u32(wimg);
+    const uint32_t wbase = smem_u32(smem);
     uint64_t *bar = &mbar[wg];
     uint32_t phase = 0;
-    bool failed = false;  // uniform over the warpgroup (decided through bar.red.and)
+    bool loaded = false;  // the weight images have arrived
+    bool ok = true;       // this thread's waits came through; the warpgroup agrees on it at its barrier
+    bool failed = false;  // uniform over the warpgroup
 
     const uint64_t ntiles = (a.count + TM - 1) / TM;
-    for (uint64_t tile = (uint64_t)blockIdx.x * kFwdWG + wg; tile < ntiles && !failed;
+    // the workload encoder's input row, loaded a tile ahead (its DRAM latency is a sixth of a tile)
+    float xr[kNrcC4Dims];
+    auto load_x = [&](uint64_t tl) {
+        const uint64_t r = tl * TM + t;
+        const bool v = a.c4 && tl < ntiles && r < a.count;
+        const float *p = a.input + r * kNrcC4Dims;
+#pragma unroll
+        for (int d = 0; d < kNrcC4Dims; d++) xr[d] = v ? ld_early(p + d) : 0.0f;
+    };
+    load_x(blockIdx.x + (uint64_t)gridDim.x * wg);
+    // one tile per SM before any SM gets a second
+    for (uint64_t tile = blockIdx.x + (uint64_t)gridDim.x * wg; tile < ntiles && !failed;
          tile += (uint64_t)gridDim.x * kFwdWG) {
         const uint64_t row = tile * TM + t;
         {
             uint32_t q[kNrcWidth / 2];
-            encode_any_pack(a.plan, a.c4 != 0, row < a.count ? a.input + row * a.n.in_dims : nullptr, q);
+            if (a.c4) {
+                encode_c4_pack(xr, row < a.count, q);
+                load_x(tile + (uint64_t)gridDim.x * kFwdWG);
+            } else {
+                encode_row_pack(a.plan, row < a.count ? a.input + row * a.n.in_dims : nullptr, q);
+            }
             tmem_st32(areg + lane_off, q);
         }
+        if (!loaded) {
+            ok = mbar_wait(&wbar, 0, a.status);
+            loaded = true;
+        }
         fence_before();
-        wg_sync(bar_id);
-        for (int l = 0; l <= L; l++) {
+        failed = !wg_sync_and(bar_id, ok);
+        for (int l = 0; l <= L && !failed; l++) {
             const bool out_layer = l == L;
-            if (t == 0) {
+            if ((warp & 3) == 0 && elect_one()) {
                 fence_after();
                 const uint32_t wl = wbase + (uint32_t)l * W * W * 2u;
                 const uint32_t idesc = out_layer ? idesc_bf16(TM, kNrcOutPad) : idesc_bf16(TM, W);
@@ -232,11 +255,7 @@ __global__ void __launch_bounds__(128 * kFwdWG, 1) k_nrc_fwd_tc(const TcArgs a) 
                     mma_bf16_ts(tmem, areg + 8u * kk, make_desc(wl + kk * 256u), idesc, kk > 0 ? 1u : 0u);
                 mma_commit(bar);
             }
-            const bool got = mbar_wait(bar, phase, a.status);
-            if (!wg_sync_and(bar_id, got)) {
-                failed = true;
-                break;
-            }
+            ok = mbar_wait(bar, phase, a.status) && ok;
             phase ^= 1u;
             fence_after();
             if (!out_layer) {
@@ -258,7 +277,7 @@ __global__ void __launch_bounds__(128 * kFwdWG, 1) k_nrc_fwd_tc(const TcArgs a) 
                     for (int c = 0; c < a.n.out_dims; c++) a.output[row * a.n.out_dims + c] = v[c];
             }
             fence_before();
-            wg_sync(bar_id);
+            failed = !wg_sync_and(bar_id, ok);
         }
     }
     if (failed) {
@@ -266,6 +285,7 @@ __global__ void __launch_bounds__(128 * kFwdWG, 1) k_nrc_fwd_tc(const TcArgs a) 
         // the accumulator columns are released
         mbar_wait(bar, phase, a.status);
     }
+    if (!loaded) mbar_wait(&wbar, 0, a.status);  // no copy in flight when the block ends
     fence_before();
     __syncthreads();
     fence_after();
@@ -290,7 +310,7 @@ struct TrainArgs {
     int c4;
     const uint16_t *wimg;
     uint32_t B;
-    const float *input, *target;
+    NrcRows rows;
     float *part;  // [gridDim.x][np]
     size_t np;
     float *loss;
@@ -356,7 +376,8 @@ __global__ void __launch_bounds__(128, 1) k_nrc_train_tc(const TrainArgs a) {
     for (uint32_t tile = blockIdx.x; tile < ntiles && !failed; tile += gridDim.x) {
         const uint32_t row = tile * TM + tid;
         const bool valid = row < a.B;
-        encode_any(a.n, a.plan, a.c4 != 0, valid ? a.input + (size_t)row * a.n.in_dims : nullptr, acts, tid);
+        const uint64_t src = valid ? a.rows.index(row) : 0;
+        encode_any(a.n, a.plan, a.c4 != 0, valid ? a.rows.input + src * a.n.in_dims : nullptr, acts, tid);
         publish();
         // ---- forward
         for (int l = 0; l <= L && !failed; l++) {
@@ -400,7 +421,7 @@ __global__ void __launch_bounds__(128, 1) k_nrc_train_tc(const TrainArgs a) {
                 for (int c = 0; c < 16; c++) {
                     gr[c] = 0.0f;
                     if (valid && c < O) {
-                        const float p = v[c], t = a.target[(size_t)row * O + c];
+                        const float p = v[c], t = a.rows.target[src * O + c];
                         const float den = p * p + 0.01f;
                         lsum += (p - t) * (p - t) / den;
                         gr[c] = 2.0f * (p - t) / den * norm;
@@ -552,13 +573,6 @@ __host__ __device__ inline uint32_t ws_slot_bytes(int L) { return (uint32_t)ws_i
 __device__ __forceinline__ uint32_t g_off(uint32_t row, uint32_t kb) {  // 8 columns kb*8.. of row
     return ((row >> 3) * 2u + kb) * 128u + (row & 7u) * 16u;
 }
-// a global load issued where it is written (an asm volatile is not moved past the other volatile
-// asm of the step loop), so its latency overlaps the steps before the value's first use
-__device__ __forceinline__ float ld_early(const float *p) {
-    float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -568,7 +582,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_nrc_train_ws(const TrainArgs 
     __shared__ uint64_t done[2], ready[2];
     __shared__ uint32_t tmem_slot;
     __shared__ float red[8];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = (int)uniform(threadIdx.x >> 5), lane = tid & 31;
     const int L = a.n.layers, O = a.n.out_dims, nimg = ws_images(L);
     const uint32_t wbytes = (uint32_t)(L * W * W + kNrcOutPad * W) * 2u;
     uint8_t *wimg = smem;
@@ -592,7 +606,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_nrc_train_ws(const TrainArgs 
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = uniform(tmem_slot);
     const uint32_t wbase = smem_u32(wimg), sbase = smem_u32(slots);
     const uint32_t wout = wbase + (uint32_t)L * W * W * 2u;
     const uint32_t c_dw = 128u, c_out = 128u + 64u * (uint32_t)L;
@@ -604,7 +618,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_nrc_train_ws(const TrainArgs 
 
     if (warp >= 8) {
         // ---- MMA issuers: warp 8 + s forward + dH of slot s, warp 10 the weight gradients
-        if (lane == 0) {
+        if (elect_one()) {
             const bool wgrad = warp == 10;
             const int own = warp - 8;  // the forward issuer's slot
             uint32_t rph[2] = {0u, 0u}, narr[2] = {0u, 0u};
@@ -693,18 +707,18 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_nrc_train_ws(const TrainArgs 
         };
         auto row_of = [&](uint32_t i) { return (blockIdx.x + i * gridDim.x) * TM + (uint32_t)r; };
         // input rows (workload encoder) and targets, loaded a tile ahead; q = the tile's packed encoding
-        float xr[kC4Dims], tr[kNrcOutPad];
+        float xr[kNrcC4Dims], tr[kNrcOutPad];
         uint32_t q[kNrcWidth / 2];
         auto valid_row = [&](uint32_t i) { return i < nt && row_of(i) < a.B; };
         auto load_x = [&](uint32_t i) {
             const bool v = c4 && valid_row(i);
-            const float *p = a.input + (size_t)row_of(i) * kC4Dims;
+            const float *p = a.rows.input + (v ? a.rows.index(row_of(i)) : 0) * kNrcC4Dims;
 #pragma unroll
-            for (int d = 0; d < kC4Dims; d++) xr[d] = v ? ld_early(p + d) : 0.0f;
+            for (int d = 0; d < kNrcC4Dims; d++) xr[d] = v ? ld_early(p + d) : 0.0f;
         };
         auto load_t = [&](uint32_t i) {
             const bool v = valid_row(i);
-            const float *p = a.target + (size_t)row_of(i) * O;
+            const float *p = a.rows.target + (v ? a.rows.index(row_of(i)) : 0) * O;
 #pragma unroll
             for (int c = 0; c < kNrcOutPad; c++) tr[c] = (v && c < O) ? ld_early(p + c) : 0.0f;
         };
@@ -719,7 +733,7 @@ __global__ void __launch_bounds__(kWsThreads, 1) k_nrc_train_ws(const TrainArgs 
         for (uint32_t i = (uint32_t)s; i < nt && !failed; i += 2) {
             const uint32_t row = row_of(i);
             const bool valid = row < a.B;
-            const float *xin = valid ? a.input + (size_t)row * a.n.in_dims : nullptr;
+            const float *xin = valid ? a.rows.input + a.rows.index(row) * a.n.in_dims : nullptr;
             encode0(valid, xin);
             publish();
             for (int k = 0; k < nsteps; k++) {
@@ -889,7 +903,7 @@ sty_status nrc_tc_forward(const NrcNet &n, const uint16_t *img, uint64_t count, 
     TcArgs a;
     a.n = n;
     a.plan = make_plan(n);
-    a.c4 = is_c4(n) ? 1 : 0;
+    a.c4 = nrc_is_c4(n) ? 1 : 0;
     a.wimg = img;
     a.count = count;
     a.input = input;
@@ -908,8 +922,7 @@ sty_status nrc_tc_forward(const NrcNet &n, const uint16_t *img, uint64_t count, 
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const uint64_t ntiles = (count + TM - 1) / TM;
-    const uint64_t ctas = (ntiles + kFwdWG - 1) / kFwdWG;
-    const uint64_t grid = ctas < (uint64_t)sms ? ctas : (uint64_t)sms;
+    const uint64_t grid = std::min<uint64_t>(ntiles, (uint64_t)sms);
     k_nrc_fwd_tc<<<(unsigned)grid, 128 * kFwdWG, smem, st>>>(a);
     return check_launch("k_nrc_fwd_tc");
 }
@@ -929,8 +942,7 @@ uint32_t nrc_tc_train_ctas(uint32_t B) {
     return ntiles < (uint32_t)sms ? ntiles : (uint32_t)sms;
 }
 
-sty_status nrc_tc_train(const NrcNet &n, const uint16_t *img, uint32_t B, const float *input, const float *target,
-                        float *part, size_t np, float *loss, uint32_t ctas, cudaStream_t st) {
+sty_status nrc_tc_train(const NrcNet &n, const uint16_t *img, uint32_t B, const NrcRows &rows, float *part, size_t np, float *loss, uint32_t ctas, cudaStream_t st) {
     if (n.layers > kNrcTcTrainMaxLayers) {
         set_error("tensor-core training supports at most %d hidden layers", kNrcTcTrainMaxLayers);
         return STY_ERR_ARG;
@@ -938,11 +950,10 @@ sty_status nrc_tc_train(const NrcNet &n, const uint16_t *img, uint32_t B, const 
     TrainArgs a;
     a.n = n;
     a.plan = make_plan(n);
-    a.c4 = is_c4(n) ? 1 : 0;
+    a.c4 = nrc_is_c4(n) ? 1 : 0;
     a.wimg = img;
     a.B = B;
-    a.input = input;
-    a.target = target;
+    a.rows = rows;
     a.part = part;
     a.np = np;
     a.loss = loss;

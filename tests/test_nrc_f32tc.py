@@ -1,4 +1,4 @@
-"""The FP32 cache's tensor-core kernels (three-way BF16 splits) against the FP64 oracle, at the edges of
+"""The FP32 cache's tensor-core inference (three-way BF16 splits) and its training step against the FP64 oracle, at the edges of
 their tiles and dispatch: one row, a row short of and past a 128-row tile, a second tile on an SM (the
 grid is one CTA of two tiles per SM), 1 to 8 hidden layers, 1 to 16 outputs (4 and 16 wide variants), the
 workload's frequency table and another one.
@@ -49,9 +49,12 @@ def test_inference_matches_oracle(sty, cuda, rows, layers, out, freqs):
 
 
 @pytest.mark.parametrize("rows,layers,out,freqs", [
-    (1, 5, 3, FREQS), (200, 1, 2, OTHER), (128 * 152 + 130, 2, 3, FREQS), (1000, 6, 16, FREQS), (777, 8, 5, FREQS),
+    (1, 5, 3, FREQS), (200, 1, 2, OTHER), (64 * 304 + 1, 2, 3, FREQS), (128 * 304 + 65, 2, 3, FREQS), (1000, 6, 16, FREQS),
+    (777, 8, 5, FREQS),
 ])
 def test_gradient_matches_oracle(sty, cuda, rows, layers, out, freqs):
+    """The CUDA-core training kernels at 64- and 128-sample tiles (the wider ones past two tiles per SM, where
+    the weights leave room), 32-row groups and quadrants of the weight gradient cut short."""
     net = _net(sty, freqs, out, layers)
     rng = np.random.default_rng(rows)
     x, t = rng.random((rows, len(freqs))).astype(np.float32), (rng.random((rows, out)) + 0.1).astype(np.float32)
@@ -60,6 +63,20 @@ def test_gradient_matches_oracle(sty, cuda, rows, layers, out, freqs):
                                 layers, out)
     assert np.linalg.norm(g.cpu().numpy() - rg) <= TOL * np.linalg.norm(rg)
     assert abs(loss - rl) <= TOL * abs(rl)
+    assert sty.abi.device_status() == 0
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_sampled_batch_is_the_gathered_one(sty, cuda, precision):
+    """A training step on rows the kernel gathers itself gives the weights of a step on the one row there is to
+    draw, repeated: count = 1, so every sample is that row (the first optimiser step is lr * sign)."""
+    import torch
+    x, t = _dev(np.random.default_rng(1).random((1, 11))), _dev([[0.3, 0.5, 0.9]])
+    nets = [sty.nrc.NRC(sty.nrc.config(FREQS, 3, 256, 3, precision, seed=4)) for _ in range(2)]
+    nets[0].train(x, t, 1)
+    nets[1].train(x.expand(256, 11).contiguous(), t.expand(256, 3).contiguous(), 1)
+    assert (nets[0].save_params() == nets[1].save_params()).all()
+    torch.cuda.synchronize()
     assert sty.abi.device_status() == 0
 
 
