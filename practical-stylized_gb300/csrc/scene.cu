@@ -1,7 +1,9 @@
-// scene.cu -- scene object: host-side binned-SAH BVH build, device upload, closest-hit queries.
+// scene.cu -- scene object: host-side binned-SAH BVH build (binary, widened to 4 children), device upload,
+// closest-hit queries.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -23,6 +25,10 @@ struct sty_scene {
     uint32_t *light_tris = nullptr;
     float *light_cdf = nullptr;
     void *render_cache = nullptr;  // device buffers of the last render, reused by the next (trace.cu)
+    // one parked device workspace, taken by a call that is given it and handed back when its work is done
+    std::mutex workspace_lock;
+    void *workspace = nullptr;
+    size_t workspace_bytes = 0;
 };
 
 namespace sty {
@@ -70,13 +76,24 @@ struct Box {
     }
 };
 
+struct Node2 {
+    float bmin[3], bmax[3];
+    uint32_t a;      // internal: left child (right = a + 1); leaf: first triangle slot
+    uint32_t count;  // 0 = internal, else number of triangles in the leaf
+    float area() const {
+        float d[3];
+        for (int k = 0; k < 3; k++) d[k] = std::max(0.0f, bmax[k] - bmin[k]);
+        return d[0] * d[1] + d[1] * d[2] + d[2] * d[0];
+    }
+};
+
 // Binned SAH (16 bins per axis), leaves of at most 4 triangles.
 struct Builder {
     const float *pos;
     std::vector<Box> tbox;
     std::vector<float> cent;  // 3 per triangle
     std::vector<uint32_t> idx;
-    std::vector<BvhNode> nodes;
+    std::vector<Node2> nodes;
 
     void build(uint32_t n) {
         tbox.resize(n);
@@ -88,10 +105,10 @@ struct Builder {
             idx[i] = i;
         }
         nodes.reserve(2 * (size_t)n);
-        nodes.push_back(BvhNode());
+        nodes.push_back(Node2());
         subdivide(0, 0, n);
     }
-    void set_bounds(BvhNode &nd, uint32_t b, uint32_t e) {
+    void set_bounds(Node2 &nd, uint32_t b, uint32_t e) {
         Box bx;
         for (uint32_t i = b; i < e; i++) bx.grow(tbox[idx[i]]);
         for (int a = 0; a < 3; a++) {
@@ -165,8 +182,8 @@ struct Builder {
             if (mid == b || mid == e) mid = b + cnt / 2;
         }
         const uint32_t l = (uint32_t)nodes.size();
-        nodes.push_back(BvhNode());
-        nodes.push_back(BvhNode());
+        nodes.push_back(Node2());
+        nodes.push_back(Node2());
         nodes[ni].a = l;
         nodes[ni].count = 0;
         subdivide(l, b, mid);
@@ -174,8 +191,82 @@ struct Builder {
     }
 };
 
+// The binary tree as 4-wide nodes (each takes its two children and opens the larger of them, by
+// surface, until it has four), the children's boxes quantised to the node's grid. Breadth first, so the
+// top of the tree is contiguous.
+std::vector<BvhNode> widen(const std::vector<Node2> &n2) {
+    std::vector<BvhNode> out(1);
+    std::vector<uint32_t> src(1, 0);  // the binary node each wide node was made from
+    out.reserve(n2.size() / 2 + 1);
+    for (size_t i = 0; i < src.size(); i++) {
+        uint32_t kid[4];
+        int nk = 0;
+        const Node2 &root = n2[src[i]];
+        if (root.count) {  // a one-leaf tree
+            kid[nk++] = src[i];
+        } else {
+            kid[nk++] = root.a;
+            kid[nk++] = root.a + 1;
+            while (nk < 4) {
+                int best = -1;
+                for (int k = 0; k < nk; k++)
+                    if (!n2[kid[k]].count && (best < 0 || n2[kid[k]].area() > n2[kid[best]].area())) best = k;
+                if (best < 0) break;
+                const uint32_t a = n2[kid[best]].a;
+                kid[best] = a;
+                kid[nk++] = a + 1;
+            }
+        }
+        BvhNode w;
+        memset(&w, 0, sizeof(w));
+        w.exp = (uint32_t)nk << 24;
+        for (int a = 0; a < 3; a++) {
+            float lo = n2[kid[0]].bmin[a], hi = n2[kid[0]].bmax[a];
+            for (int k = 1; k < nk; k++) {
+                lo = std::min(lo, n2[kid[k]].bmin[a]);
+                hi = std::max(hi, n2[kid[k]].bmax[a]);
+            }
+            if (!std::isfinite(lo) || !std::isfinite(hi)) {  // no grid holds the box: an axis that excludes nothing
+                w.o[a] = -0x1p127f;
+                w.exp |= 254u << (8 * a);
+                w.hi[a] = 0xffffffffu;
+                continue;
+            }
+            // spacing: 250 steps cover the box; not below 2^-20 of the coordinates, whose own rounding the
+            // corner has
+            const double mag = std::max(std::fabs((double)lo), std::fabs((double)hi));
+            const double need = std::max(std::max(((double)hi - lo) / 250.0, mag * 0x1p-20), 0x1p-100);
+            int e;
+            std::frexp(need, &e);  // need <= 2^e
+            const double step = std::ldexp(1.0, e);
+            w.o[a] = (float)((double)lo - 2.0 * step);
+            w.exp |= (uint32_t)(e + 127) << (8 * a);
+            for (int k = 0; k < nk; k++) {
+                const double ql = std::floor(((double)n2[kid[k]].bmin[a] - w.o[a]) / step) - 1.0;
+                const double qh = std::ceil(((double)n2[kid[k]].bmax[a] - w.o[a]) / step) + 1.0;
+                w.lo[a] |= (uint32_t)std::min(std::max(0.0, ql), 255.0) << (8 * k);
+                w.hi[a] |= (uint32_t)std::min(std::max(0.0, qh), 255.0) << (8 * k);
+            }
+        }
+        for (int k = 0; k < nk; k++) {
+            const Node2 &c = n2[kid[k]];
+            if (c.count) {
+                w.child[k] = c.a;
+                w.count |= c.count << (8 * k);
+            } else {
+                w.child[k] = (uint32_t)src.size();
+                src.push_back(kid[k]);
+                out.emplace_back();
+            }
+        }
+        out[i] = w;
+    }
+    return out;
+}
+
 void free_scene(sty_scene *s) {
     render_cache_free(s->render_cache);
+    if (s->workspace) cudaFree(s->workspace);
     void *ptrs[] = {s->nodes, s->tris, s->tri_material, s->tri_normal, s->tri_area,
                     s->tri_pos, s->materials, s->light_tris, s->light_cdf};
     for (void *p : ptrs)
@@ -279,7 +370,8 @@ sty_status sty_scene_create(const float *pos, const uint32_t *tmat, uint32_t n, 
         st = check_cuda(cudaMalloc(dst, bytes), what);
         if (st == STY_OK) st = check_cuda(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice), what);
     };
-    up((void **)&s->nodes, b.nodes.data(), b.nodes.size() * sizeof(BvhNode), "upload bvh");
+    const std::vector<BvhNode> wide = widen(b.nodes);
+    up((void **)&s->nodes, wide.data(), wide.size() * sizeof(BvhNode), "upload bvh");
     up((void **)&s->tris, tg.data(), tg.size() * sizeof(TriGeom), "upload triangles");
     up((void **)&s->tri_material, tmat, n * 4, "upload materials ids");
     up((void **)&s->tri_normal, nrm.data(), nrm.size() * 4, "upload normals");
@@ -316,6 +408,38 @@ sty_status sty_scene_closest_hit(sty_scene *s, const float *rays, uint64_t n, ui
 // accessors used by the render driver
 namespace sty {
 const sty_camera &scene_camera(const sty_scene *s) { return s->camera; }
+sty_status scene_take_workspace(sty_scene *s, size_t bytes, void **ptr, size_t *got) {
+    void *p = nullptr;
+    size_t have = 0;
+    {
+        std::lock_guard<std::mutex> g(s->workspace_lock);
+        std::swap(p, s->workspace);
+        std::swap(have, s->workspace_bytes);
+    }
+    if (p && have < bytes) {
+        cudaFree(p);
+        p = nullptr;
+    }
+    if (!p) {
+        STY_TRY(check_cuda(cudaMalloc(&p, bytes), "alloc scene workspace"));
+        have = bytes;
+    }
+    *ptr = p;
+    *got = have;
+    return STY_OK;
+}
+void scene_give_workspace(sty_scene *s, void *p, size_t bytes) {
+    constexpr size_t kKeep = (size_t)8 << 30;
+    if (bytes <= kKeep) {
+        std::lock_guard<std::mutex> g(s->workspace_lock);
+        if (!s->workspace) {
+            s->workspace = p;
+            s->workspace_bytes = bytes;
+            return;
+        }
+    }
+    cudaFree(p);
+}
 void *&scene_render_cache(sty_scene *s) { return s->render_cache; }
 void scene_bounds(const sty_scene *s, float mn[3], float mx[3]) {
     for (int a = 0; a < 3; a++) {

@@ -212,10 +212,17 @@ struct CamArgs {
 
 // One light sample for a vertex at p (sample_light, lm_path_filtering.rs:1261-1316): emitter chosen
 // by the area x luminance CDF, uniform point on it, Li styled at depth + 1 by the emitter's program
-// (flags = the vertex's updated flags), shadow ray. Returns false when the sample carries nothing.
-__device__ bool nee_sample(const SceneView &sc, F3 p, F3 ng, uint32_t prim, uint32_t new_flags, uint32_t depth,
-                           const sty_style_program *progs, uint32_t n_progs, sty_pcg32 &st, F3 *wi_out, f3 *li_out,
-                           float *pdf_out) {
+// (flags = the vertex's updated flags). Returns false when the sample carries nothing; else it carries li
+// unless the shadow ray from `so` along `wi` up to `tmax` meets a triangle other than the vertex's and `lt`.
+struct NeeSample {
+    F3 wi, so;
+    f3 li;
+    float pdf, tmax;
+    uint32_t lt;
+};
+__device__ __forceinline__ bool nee_candidate(const SceneView &sc, F3 p, F3 ng, uint32_t new_flags, uint32_t depth,
+                                              const sty_style_program *progs, uint32_t n_progs, sty_pcg32 &st,
+                                              NeeSample *out) {
     const float ux = next_1d(st), uy = next_1d(st), uz = next_1d(st);
     if (sc.n_lights == 0) return false;
     uint32_t lo = 0, hi = sc.n_lights - 1;
@@ -246,12 +253,25 @@ __device__ bool nee_sample(const SceneView &sc, F3 p, F3 ng, uint32_t prim, uint
         const int32_t pi = lm.style[style_index(new_flags)];
         if (pi >= 0 && (uint32_t)pi < n_progs) li = style_apply(progs[pi], depth + 1, li, f3{q.x, q.y, q.z});
     }
-    const F3 so = offset_ray_origin(p, face_forward(ng, wi));
-    const float s3[3] = {so.x, so.y, so.z}, w3[3] = {wi.x, wi.y, wi.z};
-    if (trace_any(sc, s3, w3, 0.0f, dist * (1.0f - 1e-3f), prim, lt)) return false;
-    *wi_out = wi;
-    *li_out = li;
-    *pdf_out = lpdf;
+    out->so = offset_ray_origin(p, face_forward(ng, wi));
+    out->wi = wi;
+    out->li = li;
+    out->pdf = lpdf;
+    out->tmax = dist * (1.0f - 1e-3f);
+    out->lt = lt;
+    return true;
+}
+// the same with its shadow ray: false also when the light is hidden
+__device__ bool nee_sample(const SceneView &sc, F3 p, F3 ng, uint32_t prim, uint32_t new_flags, uint32_t depth,
+                           const sty_style_program *progs, uint32_t n_progs, sty_pcg32 &st, F3 *wi_out, f3 *li_out,
+                           float *pdf_out) {
+    NeeSample n;
+    if (!nee_candidate(sc, p, ng, new_flags, depth, progs, n_progs, st, &n)) return false;
+    const float s3[3] = {n.so.x, n.so.y, n.so.z}, w3[3] = {n.wi.x, n.wi.y, n.wi.z};
+    if (trace_any(sc, s3, w3, 0.0f, n.tmax, prim, n.lt)) return false;
+    *wi_out = n.wi;
+    *li_out = n.li;
+    *pdf_out = n.pdf;
     return true;
 }
 // Surface::avg_roughness: diffuse 1, the GGX lobe its alpha (as the NL-PF paths have used it), the
@@ -375,7 +395,8 @@ __device__ __forceinline__ bool emitter_le(const SceneView &sc, const sty_scene_
         for (uint32_t k = 0; k < sc.n_lights; k++)
             if (sc.light_tris[k] == prim) sel = sc.light_cdf[k + 1] - sc.light_cdf[k];
         const F3 w = p - prev_p;
-        const float dist2 = dot(w, w);
+        // (fixed order, so that every kernel it is inlined in gives the same bits)
+        const float dist2 = __fmaf_rn(w.z, w.z, __fmaf_rn(w.x, w.x, __fmul_rn(w.y, w.y)));
         const F3 wn = w * (1.0f / sqrtf(dist2));
         const float lpdf = sel / sc.tri_area[prim] * dist2 / fmaxf(fabsf(dot(ng, wn)), 1e-6f);
         *mis = prev_pdf / (prev_pdf + lpdf);
