@@ -33,7 +33,7 @@ struct Geo {
     uint32_t res[3];
     uint32_t table;
     float r;
-    float r2max;  // largest f32 s with sqrt_rn(s) <= r: dist_f(..) <= r  <=>  dist2_f(..) <= r2max
+    float r2max;  // largest f32 s with sqrt_rn(s) <= r: dist_f(..) <= r  <=>  its radicand <= r2max
 };
 
 struct VArgs {  // device views of sty_pf_vertices
@@ -66,14 +66,6 @@ __device__ __forceinline__ float dist_f(float ax, float ay, float az, float bx, 
     s = __fadd_rn(s, __fmul_rn(dy, dy));
     s = __fadd_rn(s, __fmul_rn(dz, dz));
     return __fsqrt_rn(s);
-}
-
-// the radicand of dist_f, rounded the same way
-__device__ __forceinline__ float dist2_f(float ax, float ay, float az, float bx, float by, float bz) {
-    const float dx = __fsub_rn(ax, bx), dy = __fsub_rn(ay, by), dz = __fsub_rn(az, bz);
-    float s = __fmul_rn(dx, dx);
-    s = __fadd_rn(s, __fmul_rn(dy, dy));
-    return __fadd_rn(s, __fmul_rn(dz, dz));
 }
 
 // 27-cell walk (:61-123): dz outer, dy, dx inner; f(u) returns false to stop.
@@ -215,14 +207,23 @@ __global__ void k_ranges(const uint32_t *keys, const uint32_t *num, uint2 *range
     if (i == 0 || keys[i - 1] != k) ranges[k].x = (uint32_t)i;
     if (i + 1 == m || keys[i + 1] != k) ranges[k].y = (uint32_t)i + 1;
 }
-// bucket-ordered copies of what the walk reads per candidate: position + flags (16 B), cluster id
-__global__ void k_sorted_view(VArgs v, const uint32_t *num, const uint32_t *sorted, const uint32_t *cid, int cluster,
-                              float4 *spos, uint32_t *scid) {
+// What the walk reads per candidate, in bucket order: planes of positions and flags, so that a lane takes four
+// candidates with one load per field; cluster ids. `magic[c]` = floor((2^32 - 1) / (c + 1)), for draw_below.
+struct Sorted {
+    float *x, *y, *z;
+    uint8_t *flags;
+    uint32_t *cid, *magic;
+};
+__global__ void k_sorted_view(VArgs v, const uint32_t *num, const uint32_t *sorted, const uint32_t *cid, int cluster, Sorted o) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= *num) return;
     const uint32_t u = sorted[k];
-    spos[k] = make_float4(v.p[0][u], v.p[1][u], v.p[2][u], __uint_as_float(v.flags[u] & 15u));
-    if (cluster) scid[k] = cid[u];
+    o.x[k] = v.p[0][u];
+    o.y[k] = v.p[1][u];
+    o.z[k] = v.p[2][u];
+    o.flags[k] = (uint8_t)(v.flags[u] & 15u);
+    if (cluster) o.cid[k] = cid[u];
+    o.magic[k] = 0xffffffffu / (k + 1u);
 }
 
 // clustering: claim
@@ -307,22 +308,44 @@ __device__ __forceinline__ uint32_t pcg_output(uint64_t old) {
     return (xs >> rot) | (xs << ((~rot + 1u) & 31u));
 }
 
+// x % m for m >= 2 with magic = floor((2^32 - 1) / m): the product's high word is the quotient or one less
+__device__ __forceinline__ uint32_t draw_below(uint32_t x, uint32_t m, uint32_t magic) {
+    const uint32_t r = x - __umulhi(x, magic) * m;
+    return r >= m ? r - m : r;
+}
+// the radicand of dist_f on both lanes, each operation as an FMA that rounds like it (times 1, plus 0): as `mul` and `add` the
+// assembler contracts packed operations, which moved the threshold by an ulp
+__device__ __forceinline__ float2 radicand2(float2 ax, float2 ay, float2 az, float2 nbx, float2 nby, float2 nbz) {
+    const float2 one = make_float2(1.0f, 1.0f), zero = make_float2(0.0f, 0.0f);
+    const float2 dx = ffma2(ax, one, nbx), dy = ffma2(ay, one, nby), dz = ffma2(az, one, nbz);
+    const float2 s = ffma2(ffma2(dx, dx, zero), one, ffma2(dy, dy, zero));
+    return ffma2(s, one, ffma2(dz, dz, zero));
+}
+
 // Per-warp shared scratch for a reservoir of R neighbours: 64-bit (candidate index, vertex) keys,
 // the neighbour list, and each neighbour's BSDF frame with its wo-side terms precomputed for the
 // SMIS pdf sums.
 struct __align__(16) NbFrame {  // 64 bytes: four 16-byte shared-memory reads
-    float ns[3], ng[3], wo[3];
+    float ns[3];
+    float co;      // wo . ns; NaN for a flat diffuse frame (bit 3) whose bit 0 is not set
+    float ng[3];
     float fl;      // sign(ng . ns)
-    float co;      // wo . ns
+    float wo[3];
     float alpha;   // GGX: max(alpha, 1e-4)
     float g1;      // GGX: 1 / (1 + Lambda(co))
-    uint32_t bits; // bit 0: the wo half of check_wo_wi_valid holds; bit 1: GGX; bit 2: principled
+    uint32_t bits; // bit 0: the wo half of check_wo_wi_valid holds; bit 1: GGX; bit 2: principled;
+                   // bit 3: flat diffuse: ns = ng
     uint32_t mat;  // material index (the principled closure)
     uint32_t pad;
 };
 // rounded up to 16 bytes so that every warp's scratch starts 16-byte aligned for any R
+// (the queue of the gather, kQueue words, lies where the frames are made after it)
+constexpr uint32_t kQueue = 256;
+__host__ __device__ constexpr size_t frame_bytes(uint32_t R) {
+    return R * sizeof(NbFrame) > kQueue * 4u ? R * sizeof(NbFrame) : kQueue * 4u;
+}
 __host__ __device__ constexpr size_t warp_scratch_bytes(uint32_t R) {
-    return ((size_t)R * (sizeof(unsigned long long) + sizeof(uint32_t) + sizeof(NbFrame)) + 15u) & ~(size_t)15u;
+    return (frame_bytes(R) + (size_t)R * (sizeof(unsigned long long) + sizeof(uint32_t)) + 15u) & ~(size_t)15u;
 }
 __device__ __forceinline__ NbFrame make_frame(const sty_pf_material &m, uint32_t mi, V3 ns, V3 ng, V3 wo) {
     auto sgn = [](float x) { return x > 0.0f ? 1.0f : -1.0f; };
@@ -336,7 +359,9 @@ __device__ __forceinline__ NbFrame make_frame(const sty_pf_material &m, uint32_t
     const bool ggx = m.kind != STY_MAT_DIFFUSE;
     f.alpha = fmaxf(m.alpha, 1e-4f);
     f.g1 = ggx ? 1.0f / (1.0f + tr_lambda(f.co, f.alpha)) : 0.0f;
-    f.bits = (ok ? 1u : 0u) | (ggx ? 2u : 0u) | (bsdf::closure_kind(m.kind) ? 4u : 0u);
+    const bool flat = !ggx && !bsdf::closure_kind(m.kind) && f.fl > 0.0f && ns.x == ng.x && ns.y == ng.y && ns.z == ng.z;
+    f.bits = (ok ? 1u : 0u) | (ggx ? 2u : 0u) | (bsdf::closure_kind(m.kind) ? 4u : 0u) | (flat ? 8u : 0u);
+    if (flat && !ok) f.co = __int_as_float(0x7fffffff);
     f.mat = mi;
     f.pad = 0;
     return f;
@@ -369,17 +394,50 @@ __device__ __forceinline__ float frame_pdf(const NbFrame &f, V3 wi, const bsdf::
     return ok2 ? p : 0.0f;
 }
 
+// frame_pdf of four flat diffuse frames, added in order. With ns = ng the two sides of wi agree, and what is left of
+// the validity test is co ci >= 0. |ci| / pi is formed by Markstein's correction (q = x r, q + (x - q y) r with
+// r = RN(1 / y): correctly rounded where nothing underflows or overflows, checked for every significand), so
+// it has the division's bits; outside [2^-100, 2^100) the division itself is taken.
+__device__ __forceinline__ float add_flat4(const NbFrame *f, V3 wi, float sum) {
+    const float rpi = 1.0f / kPi;
+    float ci[4], p[4];
+    bool ok[4];
+    bool rare = false;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float4 a = *reinterpret_cast<const float4 *>(f + i);
+        ci[i] = dot3(wi, V3{a.x, a.y, a.z});
+        ok[i] = a.w * ci[i] >= 0.0f;
+        ci[i] = fabsf(ci[i]);
+        rare = rare || __float_as_uint(ci[i]) - (27u << 23) >= (200u << 23);
+        const float q = __fmul_rn(ci[i], rpi);
+        p[i] = __fmaf_rn(__fmaf_rn(-q, kPi, ci[i]), rpi, q);
+    }
+    if (rare)
+#pragma unroll
+        for (int i = 0; i < 4; i++) p[i] = ci[i] / kPi;
+#pragma unroll
+    for (int i = 0; i < 4; i++) sum += ok[i] ? p[i] : 0.0f;
+    return sum;
+}
+
 // One warp per active vertex (evaluate_filtered_radiance, :758-972); persistent warps take the
 // vertices in bucket order from a work counter, so that warps running together walk the same cells.
-// Gather: the 27-cell walk in the sequential order (cells dz, dy, dx; bucket entries ascending),
-// 32 candidates at a time from the bucket-ordered positions; a passing candidate's index c in that
-// order comes from a ballot prefix count. The reservoir (:806-829) keeps the first R candidates and
-// lets candidate c >= R replace slot j = pcg32() % (c + 1) when j < R, the draw being the
-// (c - R)-th of the vertex's stream. The replacing candidates of one chunk take consecutive draws,
-// so lane r's state is A^r s + inc * (1 + A + ... + A^(r-1)) from the chunk's starting state s,
-// with (A^r, sum) held by lane r; slot j keeps the largest replacing c (64-bit atomicMax of
-// (c, vertex)), which is what the sequential loop leaves there. Neighbour counts, lists and the
-// final RNG state are therefore bit-identical to the sequential walk.
+// Gather: the 27-cell walk in the sequential order (cells dz, dy, dx; bucket entries ascending), 128
+// candidates a step, four neighbouring ones per lane. Passing candidates go to a queue in that order
+// (ballots of the lanes' counts) and are taken from it 32 at a time, candidate cnt + l by lane l. The
+// reservoir (:806-829) keeps the first R candidates and lets candidate c >= R replace slot j = pcg32() % (c + 1)
+// when j < R, the draw being the (c - R)-th of the vertex's stream: a lane takes every 32nd draw, so its
+// state moves by A^32 s + inc * (1 + A + ... + A^31) from one to the next. Slot j keeps the largest
+// replacing c (64-bit atomicMax of (c, vertex)), which is what the sequential loop leaves there. Neighbour
+// counts, lists and the final RNG state are therefore bit-identical to the sequential walk.
+// Bound by instruction issue (0.72 of a scheduler's slots) and by the latency of the candidates' loads (13
+// bytes each, mostly from L2). Cornell box, 256 x 256 x 16 paths, 6 depths, radius 0.05, 64 neighbours: a render
+// of 131.5 ms with a 32-candidate step that drew where it tested, 96.7 with the queue and flat frames
+// apart (the draws' lanes are full: 35 % passed), 86.0 with four candidates per lane and the draws'
+// remainders by table, 68.3 without idle lanes on the rare division. Of these about 32 are the tests,
+// 13 the draws, 6 the pdf sums. Loading a step ahead: 6 % slower (spills); blocks taking 8 neighbouring
+// vertices at once: 11 % slower; 5 blocks per SM 4 % slower.
 // Evaluate: lanes take neighbours t = lane, lane + 32, ...; the SMIS pdf sums (:886-939) read the
 // reservoir's frames from shared memory (warp-wide broadcasts); lane sums are combined by a
 // shuffle tree, then lane 0 applies the style node and writes the vertex's radiance.
@@ -392,7 +450,7 @@ __device__ __forceinline__ uint64_t shfl64(uint64_t x, int src) {
 template <bool PRINC>
 __global__ void __launch_bounds__(256, 4) k_ref_filter(VArgs v, Geo g, const uint32_t *num, uint32_t *next,
                                                     const uint2 *ranges,
-                                                    const uint32_t *sorted, const float4 *spos, const uint32_t *scid,
+                                                    const uint32_t *sorted, Sorted so,
                                                     const uint32_t *cid, const float *in_next, sty_pf_ref_params prm,
                                                     const sty_pf_material *mats, uint32_t n_mats,
                                                     const bsdf::PClosure *cls, const float *tab,
@@ -405,14 +463,20 @@ __global__ void __launch_bounds__(256, 4) k_ref_filter(VArgs v, Geo g, const uin
     uint8_t *ws = smem_raw + (size_t)wib * warp_scratch_bytes(R);
     // frames first (16-byte aligned), then the 8-byte keys, then the list
     NbFrame *frames = reinterpret_cast<NbFrame *>(ws);
-    unsigned long long *keys = reinterpret_cast<unsigned long long *>(ws + (size_t)R * sizeof(NbFrame));
-    uint32_t *list = reinterpret_cast<uint32_t *>(ws + (size_t)R * (sizeof(NbFrame) + sizeof(unsigned long long)));
+    unsigned long long *keys = reinterpret_cast<unsigned long long *>(ws + frame_bytes(R));
+    uint32_t *list = reinterpret_cast<uint32_t *>(ws + frame_bytes(R) + (size_t)R * sizeof(unsigned long long));
+    uint32_t *queue = reinterpret_cast<uint32_t *>(ws);
     const unsigned lt_mask = (1u << lane) - 1u;
-    // lane r: A^r and 1 + A + ... + A^(r-1) (mod 2^64), for the reservoir draws
-    uint64_t a_pow = 1u, a_sum = 0u;
-    for (int r = 0; r < lane; r++) {
-        a_sum += a_pow;
-        a_pow *= 0x5851f42d4c957f2dULL;
+    // For the reservoir draws, A^d and 1 + A + ... + A^(d-1) (mod 2^64) with d = (lane - R) mod 32, the first draw
+    // this lane takes, and the same for d = 32, the draws between two of its.
+    uint64_t a_pow = 1u, a_sum = 0u, a32 = 1u, s32 = 0u;
+    for (uint32_t r = 0, d = (lane - R) & 31u; r < 32; r++) {
+        if (r == d) {
+            a_pow = a32;
+            a_sum = s32;
+        }
+        s32 += a32;
+        a32 *= 0x5851f42d4c957f2dULL;
     }
     const uint32_t nact = *num;
     for (;;) {
@@ -429,7 +493,8 @@ __global__ void __launch_bounds__(256, 4) k_ref_filter(VArgs v, Geo g, const uin
     const uint32_t my_cluster = prm.cluster ? cid[vi] : NONE;
     const uint32_t my_flags = v.flags[vi] & 15u;
     const sty_pcg32 st0 = rng[vi];
-    uint64_t s_cur = st0.state;  // state before the next draw (warp-uniform)
+    uint64_t s_next = a_pow * st0.state + a_sum * st0.inc, s_last = 0u;  // states before this lane's next and last draw
+    const uint64_t inc32 = s32 * st0.inc;
     // lane l < 27 looks up cell l of the walk order (dz outer, dy, dx inner)
     uint2 my_rg = make_uint2(0u, 0u);
     {
@@ -443,63 +508,91 @@ __global__ void __launch_bounds__(256, 4) k_ref_filter(VArgs v, Geo g, const uin
         }
     }
     // ---- gather
-    uint32_t cnt = 0;  // warp-uniform
+    const uint32_t flag_mask = prm.disable_flag_check ? 0u : 0x0f0f0f0fu, want_flags = my_flags * 0x01010101u;
+    const float2 nqx = make_float2(-qx, -qx), nqy = make_float2(-qy, -qy), nqz = make_float2(-qz, -qz);
+    uint32_t cnt = 0, queued = 0;  // candidates taken, candidates waiting in `queue` behind them (warp-uniform)
+    // the next `nb` candidates of the queue (32, fewer only at the end), candidate cnt + l by lane l
+    auto take = [&](uint32_t nb) {
+        const uint32_t c = cnt + lane;
+        const bool have = lane < (int)nb;
+        const uint32_t kk = have ? queue[c % kQueue] : 0u;
+        if (have && c < R) keys[c] = ((unsigned long long)c << 32) | sorted[kk];
+        __syncwarp();
+        if (have && c >= R) {
+            const uint32_t j = draw_below(pcg_output(s_next), c + 1u, so.magic[c]);
+            if (j < R) atomicMax(&keys[j], ((unsigned long long)c << 32) | sorted[kk]);
+            s_last = s_next;
+            s_next = a32 * s_next + inc32;
+        }
+        cnt += nb;
+        queued -= nb;
+    };
     for (int cell = 0; cell < 27; cell++) {
-                const uint2 rg = make_uint2(__shfl_sync(0xffffffffu, my_rg.x, cell), __shfl_sync(0xffffffffu, my_rg.y, cell));
-                // four chunks of 32 candidates per step: their loads are issued together
-                for (uint32_t base = rg.x; base < rg.y; base += 128) {
-                    float4 e[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const uint32_t kk = base + q * 32 + lane;
-                        e[q] = kk < rg.y ? spos[kk] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        if (base + q * 32 >= rg.y) break;  // warp-uniform
-                        const uint32_t kk = base + q * 32 + lane;
-                        bool pass = false;
-                        if (kk < rg.y) {
-                            pass = dist2_f(e[q].x, e[q].y, e[q].z, qx, qy, qz) <= g.r2max;
-                            if (pass && prm.cluster && scid[kk] != my_cluster) pass = false;
-                            if (pass && !prm.disable_flag_check && __float_as_uint(e[q].w) != my_flags) pass = false;
-                        }
-                        const unsigned bal = __ballot_sync(0xffffffffu, pass);
-                        if (bal == 0u) continue;
-                        const uint32_t c = cnt + __popc(bal & lt_mask);
-                        const uint32_t u = pass ? sorted[kk] : 0u;
-                        if (pass && c < R) keys[c] = ((unsigned long long)c << 32) | u;
-                        __syncwarp();
-                        const bool rep = pass && c >= R;
-                        const unsigned balr = __ballot_sync(0xffffffffu, rep);
-                        if (balr) {
-                            const int r = __popc(balr & lt_mask);
-                            const uint64_t ap = shfl64(a_pow, r), as = shfl64(a_sum, r);
-                            const uint64_t s_m = ap * s_cur + st0.inc * as;
-                            if (rep) {
-                                const uint32_t j = pcg_output(s_m) % (c + 1u);
-                                if (j < R) atomicMax(&keys[j], ((unsigned long long)c << 32) | u);
-                            }
-                            const int last = 31 - __clz((int)balr);
-                            s_cur = shfl64(s_m * 0x5851f42d4c957f2dULL + st0.inc, last);
-                        }
-                        __syncwarp();
-                        cnt += __popc(bal);
-                    }
-                }
+        const uint2 rg = make_uint2(__shfl_sync(0xffffffffu, my_rg.x, cell), __shfl_sync(0xffffffffu, my_rg.y, cell));
+        // 128 candidates per step, 4 l .. 4 l + 3 by lane l
+        for (uint32_t base = rg.x & ~3u; base < rg.y; base += 128) {
+            const uint32_t i0 = base + 4 * lane;
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x, z = x;
+            uint32_t fl = 0u;
+            if (i0 < rg.y) {
+                x = *reinterpret_cast<const float4 *>(so.x + i0);
+                y = *reinterpret_cast<const float4 *>(so.y + i0);
+                z = *reinterpret_cast<const float4 *>(so.z + i0);
+                fl = *reinterpret_cast<const uint32_t *>(so.flags + i0);
             }
+            const float2 da = radicand2(make_float2(x.x, x.y), make_float2(y.x, y.y), make_float2(z.x, z.y), nqx, nqy, nqz);
+            const float2 db = radicand2(make_float2(x.z, x.w), make_float2(y.z, y.w), make_float2(z.z, z.w), nqx, nqy, nqz);
+            fl = (fl ^ want_flags) & flag_mask;
+            uint32_t m = (da.x <= g.r2max && !(fl & 0xffu) ? 1u : 0u) | (da.y <= g.r2max && !(fl & 0xff00u) ? 2u : 0u) |
+                         (db.x <= g.r2max && !(fl & 0xff0000u) ? 4u : 0u) | (db.y <= g.r2max && !(fl & 0xff000000u) ? 8u : 0u);
+            if (base < rg.x || base + 128u > rg.y) {  // the ends of the cell
+                const uint32_t lo = rg.x > i0 ? min(rg.x - i0, 4u) : 0u, hi = rg.y > i0 ? min(rg.y - i0, 4u) : 0u;
+                m &= ((1u << hi) - 1u) & ~((1u << lo) - 1u);
+            }
+            if (prm.cluster && m) {
+                const uint4 ci = *reinterpret_cast<const uint4 *>(so.cid + i0);
+                m &= (ci.x == my_cluster ? 1u : 0u) | (ci.y == my_cluster ? 2u : 0u) | (ci.z == my_cluster ? 4u : 0u) |
+                     (ci.w == my_cluster ? 8u : 0u);
+            }
+            const uint32_t nm = __popc(m);
+            const unsigned b0 = __ballot_sync(0xffffffffu, nm & 1u), b1 = __ballot_sync(0xffffffffu, nm & 2u),
+                           b2 = __ballot_sync(0xffffffffu, nm & 4u);
+            if (!(b0 | b1 | b2)) continue;
+            uint32_t at = cnt + queued + __popc(b0 & lt_mask) + 2u * __popc(b1 & lt_mask) + 4u * __popc(b2 & lt_mask);
+#pragma unroll
+            for (uint32_t q = 0; q < 4; q++)
+                if ((m >> q) & 1u) queue[at++ % kQueue] = i0 + q;
+            queued += __popc(b0) + 2u * __popc(b1) + 4u * __popc(b2);
+            __syncwarp();
+#pragma unroll 1
+            while (queued >= 32u) take(32u);
+        }
+    }
+    if (queued) take(queued);
+    __syncwarp();
+    const uint64_t s_end = shfl64(s_last * 0x5851f42d4c957f2dULL + st0.inc, (int)((cnt - 1u) & 31u));
     if (lane == 0) {
         sty_pcg32 st = st0;
-        st.state = s_cur;
+        if (cnt > R) st.state = s_end;
         rng[vi] = st;
         if (neighbours) neighbours[vi] = cnt;
     }
     const uint32_t k = min(cnt, R);
-    for (uint32_t t = lane; t < k; t += 32) {
-        const uint32_t u = (uint32_t)keys[t];
-        list[t] = u;
-        const uint32_t mu = min(v.material[u], n_mats - 1);
-        frames[t] = make_frame(mats[mu], mu, ld3(v.ns, u), ld3(v.ng, u), ld3(v.wo, u));
+    const uint32_t rounds = (k + 31u) / 32u;  // every lane runs the SMIS loop the same number of times
+    uint32_t flat = 0;  // lane r: which of neighbours 32 r .. 32 r + 31 have flat diffuse frames
+    for (uint32_t r = 0; r < rounds; r++) {
+        const uint32_t t = r * 32u + lane;
+        bool fl = false;
+        if (t < k) {
+            const uint32_t u = (uint32_t)keys[t];
+            list[t] = u;
+            const uint32_t mu = min(v.material[u], n_mats - 1);
+            const NbFrame f = make_frame(mats[mu], mu, ld3(v.ns, u), ld3(v.ng, u), ld3(v.wo, u));
+            frames[t] = f;
+            fl = (f.bits & 8u) != 0u;
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, fl);
+        if (lane == (int)r) flat = bal;
     }
     __syncwarp();
 
@@ -510,7 +603,6 @@ __global__ void __launch_bounds__(256, 4) k_ref_filter(VArgs v, Geo g, const uin
     const V3 wo = ld3(v.wo, vi), ns = ld3(v.ns, vi), ng = ld3(v.ng, vi);
     float direct[3] = {0.f, 0.f, 0.f}, indirect[3] = {0.f, 0.f, 0.f};
     const float invk = k ? 1.0f / (float)k : 0.0f;
-    const uint32_t rounds = (k + 31u) / 32u;  // every lane runs the SMIS loop the same number of times
     for (uint32_t r = 0; r < rounds; r++) {
         const uint32_t t = r * 32u + lane;
         const bool have = t < k;
@@ -537,20 +629,22 @@ __global__ void __launch_bounds__(256, 4) k_ref_filter(VArgs v, Geo g, const uin
                 for (int c = 0; c < 3; c++) reused[c] = f[c] * (in_next ? in_next[c * n + u] : 0.0f) * mis;
             }
         }
+        // a lane whose sum is not used takes some direction that keeps its warp off the rare path of add_flat4
+        if (!ind) wi = {0.6f, 0.5f, 0.62f};
         if (prm.smis) {
             float sum_pdf = 0.0f;
-            uint32_t a = 0;
-            for (; a + 4 <= k; a += 4) {
-                const float p0 = frame_pdf<PRINC>(frames[a], wi, cls, tab);
-                const float p1 = frame_pdf<PRINC>(frames[a + 1], wi, cls, tab);
-                const float p2 = frame_pdf<PRINC>(frames[a + 2], wi, cls, tab);
-                const float p3 = frame_pdf<PRINC>(frames[a + 3], wi, cls, tab);
-                sum_pdf += p0;  // in list order, as the sequential sum
-                sum_pdf += p1;
-                sum_pdf += p2;
-                sum_pdf += p3;
+            // in list order, as the sequential sum
+            uint32_t word = 0;
+#pragma unroll 1
+            for (uint32_t a = 0; a < k; a += 4) {
+                if ((a & 31u) == 0u) word = __shfl_sync(0xffffffffu, flat, (int)(a >> 5));
+                if ((word & 15u) == 15u)
+                    sum_pdf = add_flat4(frames + a, wi, sum_pdf);
+                else
+#pragma unroll 1
+                    for (uint32_t b = a; b < min(a + 4u, k); b++) sum_pdf += frame_pdf<PRINC>(frames[b], wi, cls, tab);
+                word >>= 4;
             }
-            for (; a < k; a++) sum_pdf += frame_pdf<PRINC>(frames[a], wi, cls, tab);
             if (ind && sum_pdf > 0.0f)
 #pragma unroll
                 for (int c = 0; c < 3; c++) indirect[c] += reused[c] / sum_pdf;
@@ -595,8 +689,8 @@ struct sty_pf_ref_ctx {
     uint2 *ranges = nullptr;
     uint32_t *cid = nullptr, *csize = nullptr, *size0 = nullptr, *prop = nullptr, *winner = nullptr;
     uint32_t *counter = nullptr;
-    float4 *spos = nullptr;  // bucket-ordered position + flags
-    uint32_t *scid = nullptr;  // bucket-ordered cluster id
+    char *view = nullptr;  // the planes of Sorted, each of `plane` = cap rounded up to 4 elements, but for magic
+    size_t plane = 0;
     sty_pf_material *mats = nullptr;      // device copies of the host tables
     sty::bsdf::PClosure *cls = nullptr;   // principled closures of the materials (host-built)
     std::vector<sty::bsdf::PClosure> hcls;  // their host copy (the async upload's source)
@@ -612,7 +706,7 @@ namespace {
 void free_ctx(sty_pf_ref_ctx *c) {
     void *ptrs[] = {c->act,   c->num,    c->keys,  c->vals,    c->keys_s,  c->vals_s, c->ranges, c->cid,
                     c->csize, c->size0,  c->prop,  c->winner,  c->counter, c->mats,   c->progs,  c->tmp,
-                    c->spos,  c->scid,   c->cls};
+                    c->view,  c->cls};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     delete c;
@@ -677,8 +771,8 @@ sty_status sty_pf_ref_create(uint64_t max_vertices, uint32_t table_size, sty_pf_
     alloc((void **)&c->prop, n * 4, "alloc prop");
     alloc((void **)&c->winner, (size_t)table_size * 4, "alloc winner");
     alloc((void **)&c->counter, 4, "alloc counter");
-    alloc((void **)&c->spos, n * sizeof(float4), "alloc sorted positions");
-    alloc((void **)&c->scid, n * 4, "alloc sorted cluster ids");
+    c->plane = (n + 3) & ~(size_t)3;
+    alloc((void **)&c->view, c->plane * 17, "alloc sorted view");
     alloc((void **)&c->mats, kMaxMaterials * sizeof(sty_pf_material), "alloc materials");
     alloc((void **)&c->cls, kMaxMaterials * sizeof(bsdf::PClosure), "alloc closures");
     alloc((void **)&c->progs, kMaxPrograms * sizeof(sty_style_program), "alloc programs");
@@ -845,11 +939,14 @@ sty_status sty_pf_ref_filter(sty_pf_ref_ctx *ctx, const sty_pf_vertices *v, cons
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const uint64_t want = (n + wpb - 1) / wpb, cap_blocks = (uint64_t)std::max(per_sm, 1) * (uint64_t)std::max(sms, 1);
     const unsigned nbf = (unsigned)std::min(want, cap_blocks);
-    k_sorted_view<<<nb, bs, 0, st>>>(va, ctx->num, ctx->vals_s, ctx->cid, prm->cluster, ctx->spos, ctx->scid);
+    float *const sx = reinterpret_cast<float *>(ctx->view);
+    // (the sorted bucket keys are not read past k_ranges: magic takes their place)
+    const Sorted so = {sx, sx + ctx->plane, sx + 2 * ctx->plane, reinterpret_cast<uint8_t *>(sx + 4 * ctx->plane),
+                       reinterpret_cast<uint32_t *>(sx + 3 * ctx->plane), ctx->keys_s};
+    k_sorted_view<<<nb, bs, 0, st>>>(va, ctx->num, ctx->vals_s, ctx->cid, prm->cluster, so);
     STY_TRY(check_launch("k_sorted_view"));
     STY_TRY(check_cuda(cudaMemsetAsync(ctx->counter, 0, 4, st), "reset work counter"));
-    kern<<<nbf, 32 * wpb, smem, st>>>(va, g, ctx->num, ctx->counter, ctx->ranges, ctx->vals_s, ctx->spos,
-                                              ctx->scid, ctx->cid,
+    kern<<<nbf, 32 * wpb, smem, st>>>(va, g, ctx->num, ctx->counter, ctx->ranges, ctx->vals_s, so, ctx->cid,
                                               in_next, *prm, ctx->mats, n_materials, ctx->cls, ggx_tab, ctx->progs,
                                               n_programs, rng, out, neighbours);
     STY_TRY(check_launch("k_ref_filter"));
