@@ -340,7 +340,7 @@ STY_API sty_status sty_pf_adjoint(const sty_pf_records *rec, uint32_t depth, int
 /* Allocation-free variant of sty_pf_adjoint (no counterpart in the reference). For callers that
  * cannot allocate device memory -- a host integrator whose device memory is owned and budgeted by
  * another runtime, or a render loop that must not fail on an allocation mid-frame -- the scratch
- * lives in one fixed device array of 4.31 MiB that every device holds from the library's first use
+ * lives in one fixed device array of 4.88 MiB that every device holds from the library's first use
  * on it until the process exits. Same arguments and results as sty_pf_adjoint; limits: at most
  * 2^18 records per depth (width * height * spp), 2^16 pixels and 4096 32x8 tiles, larger inputs
  * are rejected with STY_ERR_ARG. It calls no cudaMalloc / cudaFree. Its first call on a device

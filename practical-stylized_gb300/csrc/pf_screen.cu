@@ -420,20 +420,9 @@ int32_t screen_kernel_choice() {
 
 using namespace sty;
 
-extern "C" {
-
-sty_status sty_pf_screen_set_kernel(int32_t kernel) {
-    clear_error();
-    STY_ARG_CHECK(kernel == STY_SCREEN_KERNEL_AUTO || kernel == STY_SCREEN_KERNEL_FP32 ||
-                      kernel == STY_SCREEN_KERNEL_TENSOR,
-                  "sty_pf_screen_set_kernel: unknown kernel %d", kernel);
-    g_screen_kernel.store(kernel, std::memory_order_relaxed);
-    return STY_OK;
-}
-
-sty_status sty_pf_screen_filter_depth(const sty_pf_records *rec, uint32_t depth, const sty_pf_screen_params *params,
-                                      const sty_style_program *style, const float *out_next, float *out,
-                                      float *filtered, void *stream) {
+sty_status sty::screen_filter_depth(const sty_pf_records *rec, uint32_t depth, const sty_pf_screen_params *params,
+                                    const sty_style_program *style, const float *out_next, float *out, float *filtered,
+                                    bool tensor_allowed, void *stream) {
     clear_error();
     STY_TRY(validate(rec, params));
     STY_ARG_CHECK(out, "sty_pf_screen_filter_depth: null out");
@@ -469,7 +458,7 @@ sty_status sty_pf_screen_filter_depth(const sty_pf_records *rec, uint32_t depth,
         case 1: return launch_screen<1>(a, prog, st);
         case 2: return launch_screen<2>(a, prog, st);
         case 4:  // the warp-specialised kernel's shared-memory ring fits up to radius 24
-            if (screen_kernel_choice() == STY_SCREEN_KERNEL_TENSOR && screen_tc_supports(a, 4))
+            if (tensor_allowed && screen_kernel_choice() == STY_SCREEN_KERNEL_TENSOR && screen_tc_supports(a, 4))
                 return launch_screen_tc(a, prog, st);
             return a.R <= 24 ? launch_screen_s4(a, prog, st) : launch_screen<4>(a, prog, st);
         case 8: return launch_screen<8>(a, prog, st);
@@ -482,6 +471,23 @@ sty_status sty_pf_screen_filter_depth(const sty_pf_records *rec, uint32_t depth,
                                                                   : launch_screen_g<16, 4>(a, prog, st);
         }
     }
+}
+
+extern "C" {
+
+sty_status sty_pf_screen_set_kernel(int32_t kernel) {
+    clear_error();
+    STY_ARG_CHECK(kernel == STY_SCREEN_KERNEL_AUTO || kernel == STY_SCREEN_KERNEL_FP32 ||
+                      kernel == STY_SCREEN_KERNEL_TENSOR,
+                  "sty_pf_screen_set_kernel: unknown kernel %d", kernel);
+    g_screen_kernel.store(kernel, std::memory_order_relaxed);
+    return STY_OK;
+}
+
+sty_status sty_pf_screen_filter_depth(const sty_pf_records *rec, uint32_t depth, const sty_pf_screen_params *params,
+                                      const sty_style_program *style, const float *out_next, float *out,
+                                      float *filtered, void *stream) {
+    return sty::screen_filter_depth(rec, depth, params, style, out_next, out, filtered, true, stream);
 }
 
 sty_status sty_pf_screen_filter(const sty_pf_records *rec, const sty_pf_screen_params *params,

@@ -28,6 +28,11 @@ sty_status launch_screen_s4(const ScreenArgs &a, const sty_style_program &style,
 sty_status launch_screen_s16(const ScreenArgs &a, const sty_style_program &style, cudaStream_t st);
 int screen_ws_max_radius(int spp, size_t optin);
 
+// sty_pf_screen_filter_depth, with the tensor kernel only where `tensor_allowed`
+sty_status screen_filter_depth(const sty_pf_records *rec, uint32_t depth, const sty_pf_screen_params *params,
+                               const sty_style_program *style, const float *out_next, float *out, float *filtered,
+                               bool tensor_allowed, void *stream);
+
 // tcgen05 split-TF32 kernel (pf_screen_tc.cu): 4 spp, radius 15 or 16, 16-byte aligned planes
 bool screen_tc_supports(const ScreenArgs &a, int spp);
 sty_status launch_screen_tc(const ScreenArgs &a, const sty_style_program &style, cudaStream_t st);
