@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kThreads) k_gemm_rows(const RowArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_slot;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = (int)uniform(threadIdx.x >> 5);
     const uint32_t cols = tmem_cols(a.n);
     const uint32_t wbytes = (uint32_t)a.n * a.ka * 2u, abytes = (uint32_t)TM * a.ka * 2u;
     uint8_t *wimg = smem;
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kThreads) k_gemm_rows(const RowArgs a) {
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = uniform(tmem_slot);
     const uint32_t lane_base = tmem + (((uint32_t)warp * 32u) << 16);
     const uint32_t wbase = smem_u32(wimg);
     const uint32_t sbo_k = (uint32_t)(a.ka / 8) * 128u, nstride = (uint32_t)(a.n / 8) * 128u;
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kThreads) k_gemm_rows(const RowArgs a) {
         fence_before();
         __syncthreads();
         const uint32_t abase = smem_u32(aimgs[k & 1]);
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             fence_after();
             for (int ks = 0; ks < a.ka / 16; ks++) {
                 const uint64_t ad = make_desc(abase + (uint32_t)ks * 256u, 128u, sbo_k);
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kThreads) k_gemm_dw(const DwArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t bars[2];
     __shared__ uint32_t tmem_slot;
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = (int)uniform(threadIdx.x >> 5);
     const uint32_t cols = tmem_cols(a.nq);
     const uint32_t pbytes = kDwStep * TM * 2u, qbytes = (uint32_t)kDwStep * a.nq * 2u;
     const uint32_t bufbytes = ((pbytes + qbytes) + 1023u) & ~1023u;
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(kThreads) k_gemm_dw(const DwArgs a) {
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = uniform(tmem_slot);
     const uint32_t lane_base = tmem + (((uint32_t)warp * 32u) << 16);
     const int b0 = blockIdx.x * a.chunk, b1 = min(a.rows, b0 + a.chunk);
     const int steps = b1 > b0 ? (b1 - b0 + kDwStep - 1) / kDwStep : 0;
@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kThreads) k_gemm_dw(const DwArgs a) {
         fence_async_smem();
         fence_before();
         __syncthreads();
-        if (tid == 0) {
+        if (warp == 0 && elect_one()) {
             fence_after();
             const uint32_t pb = smem_u32(pimg), qb = smem_u32(qimg);
             for (int ks = 0; ks < kDwStep / 16; ks++)
