@@ -192,10 +192,12 @@ struct Builder {
 };
 
 // The binary tree as 4-wide nodes (each takes its two children and opens the larger of them, by
-// surface, until it has four), the children's boxes quantised to the node's grid. Breadth first, so the
+// surface, until it has `width`), the children's boxes quantised to the node's grid. Breadth first, so the
 // top of the tree is contiguous.
-std::vector<BvhNode> widen(const std::vector<Node2> &n2) {
+std::vector<BvhNode> widen(const std::vector<Node2> &n2, int width, int *stack) {
     std::vector<BvhNode> out(1);
+    std::vector<int> held(1, 0);  // entries on a walk's stack at most when it comes to the node
+    *stack = 0;
     std::vector<uint32_t> src(1, 0);  // the binary node each wide node was made from
     out.reserve(n2.size() / 2 + 1);
     for (size_t i = 0; i < src.size(); i++) {
@@ -207,7 +209,7 @@ std::vector<BvhNode> widen(const std::vector<Node2> &n2) {
         } else {
             kid[nk++] = root.a;
             kid[nk++] = root.a + 1;
-            while (nk < 4) {
+            while (nk < width) {
                 int best = -1;
                 for (int k = 0; k < nk; k++)
                     if (!n2[kid[k]].count && (best < 0 || n2[kid[k]].area() > n2[kid[best]].area())) best = k;
@@ -217,6 +219,8 @@ std::vector<BvhNode> widen(const std::vector<Node2> &n2) {
                 kid[nk++] = a + 1;
             }
         }
+        const int holds = held[i] + nk - 1;
+        *stack = std::max(*stack, holds);
         BvhNode w;
         memset(&w, 0, sizeof(w));
         w.exp = (uint32_t)nk << 24;
@@ -256,6 +260,7 @@ std::vector<BvhNode> widen(const std::vector<Node2> &n2) {
             } else {
                 w.child[k] = (uint32_t)src.size();
                 src.push_back(kid[k]);
+                held.push_back(holds);
                 out.emplace_back();
             }
         }
@@ -370,7 +375,9 @@ sty_status sty_scene_create(const float *pos, const uint32_t *tmat, uint32_t n, 
         st = check_cuda(cudaMalloc(dst, bytes), what);
         if (st == STY_OK) st = check_cuda(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice), what);
     };
-    const std::vector<BvhNode> wide = widen(b.nodes);
+    // A wide node leaves up to three entries on the stack per level: a tree too deep for that gets narrower nodes.
+    std::vector<BvhNode> wide;
+    for (int width = 4, stack = kStack + 1; width >= 2 && stack > kStack; width--) wide = widen(b.nodes, width, &stack);
     up((void **)&s->nodes, wide.data(), wide.size() * sizeof(BvhNode), "upload bvh");
     up((void **)&s->tris, tg.data(), tg.size() * sizeof(TriGeom), "upload triangles");
     up((void **)&s->tri_material, tmat, n * 4, "upload materials ids");

@@ -1,4 +1,4 @@
-// scene.cuh -- device view of a scene: BVH2 nodes, triangles, materials; watertight intersection.
+// scene.cuh -- device view of a scene: 4-wide BVH nodes, triangles, materials; watertight intersection.
 #pragma once
 
 #include "common.cuh"
