@@ -362,7 +362,8 @@ STY_API sty_status sty_pf_adjoint_noalloc(const sty_pf_records *rec, uint32_t de
  * sin(2^k pi x), cos(2^k pi x), k < freqs[d]; sum 2*freqs = 64), then `hidden_layers` ReLU layers
  * of width 64 and a linear output layer of `output_dims` (<= 16); no biases. Weights are FP32
  * masters; precision STY_NRC_BF16 runs the MLP on the tcgen05 tensor cores (BF16 operands, FP32
- * accumulation in TMEM), STY_NRC_FP32 runs it in FP32 on the CUDA cores.
+ * accumulation in TMEM), STY_NRC_FP32 runs it in FP32: inference on the tensor cores as products of three-way
+ * BF16 splits (no less exact than FP32 sums), training on the CUDA cores.
  * Loss: relative L2, (pred - target)^2 / (pred^2 + 0.01) with pred treated as constant in the
  * denominator, averaged over the batch and channels. Optimiser: Adam (beta1, beta2, eps) with
  * learning rate lr * decay_base^(step / decay_interval) (tcnn ExponentialDecay, nrc_pt.rs:1199-1216);
