@@ -208,7 +208,8 @@ __global__ void k_ranges(const uint32_t *keys, const uint32_t *num, uint2 *range
     if (i + 1 == m || keys[i + 1] != k) ranges[k].y = (uint32_t)i + 1;
 }
 // What the walk reads per candidate, in bucket order: planes of positions and flags, so that a lane takes four
-// candidates with one load per field; cluster ids. `magic[c]` = floor((2^32 - 1) / (c + 1)), for draw_below.
+// candidates with one load per field; cluster ids. `magic[c]` = floor((2^32 - 1) / (c + 1)), for draw_below, with as
+// many entries as there are points.
 struct Sorted {
     float *x, *y, *z;
     uint8_t *flags;
@@ -519,7 +520,8 @@ __global__ void __launch_bounds__(256, 4) k_ref_filter(VArgs v, Geo g, const uin
         if (have && c < R) keys[c] = ((unsigned long long)c << 32) | sorted[kk];
         __syncwarp();
         if (have && c >= R) {
-            const uint32_t j = draw_below(pcg_output(s_next), c + 1u, so.magic[c]);
+            // (cells that share a bucket list its points once each: c can pass the number of points, and the table)
+            const uint32_t x = pcg_output(s_next), j = c < nact ? draw_below(x, c + 1u, so.magic[c]) : x % (c + 1u);
             if (j < R) atomicMax(&keys[j], ((unsigned long long)c << 32) | sorted[kk]);
             s_last = s_next;
             s_next = a32 * s_next + inc32;
