@@ -42,12 +42,66 @@ struct RecOut {
     uint32_t *prim;
 };
 
-// Bound by the latency of the walks' loads and by divergence: 6 blocks of 256 threads per SM (42 registers) hide
-// more of it than the spills cost. 16 paths per pixel, depth 5, with a screen filter of radius 1: room of
-// 49.6 k triangles at 512 x 384 29.2 ms on a binary tree at 104 registers, 17.3 so; Cornell box at 512 x 512
-// 11.5 and 11.1. Without the bounds (120 registers) 22.0 and 12.6.
+// Bound by the latency of the walks' loads and by divergence; how many blocks an SM should hold at the cost of spills
+// depends on how many there are (TraceJob::trace). Records of 16 paths per pixel, depth 5: room of 49.6 k triangles at
+// 512 x 384 26.2 ms on a binary tree with 104 registers, 15.1 so; Cornell box 6.2 and 5.7, of the GGX lobe 6.75 and 6.86.
+// Scenes with closures (principled, glass): the closures' code is long and its lanes few, so a walk beside it pays for its
+// registers or its spills. There (SPLIT) the walks have kernels of their own around it, k_trace_hits and
+// k_trace_shadow: principled Cornell box 10.7 ms, room 18.0; with one kernel 14.9 and 35.6 on the binary tree, 23.7 and 36.5
+// on the wide one at 40 registers, 24.9 and 45.6 at 107. Between the kernels the path's planes carry the hit (o:
+// barycentrics, triangle) and the vertex's the shadow ray (ind_wi: origin, dir_wi: direction, ind_mis: length).
 constexpr int kTraceThreads = 256;
-__global__ void __launch_bounds__(kTraceThreads, 6) k_trace(SceneView sc, CamArgs cam, uint32_t n_paths, uint32_t depth, uint32_t max_depth,
+__device__ __forceinline__ void trace_camera(const CamArgs &cam, uint32_t tid, sty_pcg32 &st, F3 *ro, F3 *rd) {
+    const uint32_t npx = cam.W * cam.H;
+    const uint32_t px = cam.random_px ? pcg_next(st) % npx : cam.pixel_major ? tid / cam.pixel_major : tid % npx;
+    camera_ray(cam, px, st, ro, rd);
+}
+__global__ void __launch_bounds__(kTraceThreads, 5) k_trace_hits(SceneView sc, CamArgs cam, uint32_t n_paths, uint32_t depth,
+                                                                 PathState ps, sty_pcg32 *rng) {
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+    if (tid >= n_paths) return;
+    F3 ro, rd;
+    uint32_t exclude = NONE;
+    if (depth == 0) {
+        sty_pcg32 st = rng[tid];
+        trace_camera(cam, tid, st, &ro, &rd);
+        rng[tid] = st;
+        ps.d[0][tid] = rd.x; ps.d[1][tid] = rd.y; ps.d[2][tid] = rd.z;
+        ps.prev_p[0][tid] = ro.x; ps.prev_p[1][tid] = ro.y; ps.prev_p[2][tid] = ro.z;
+        ps.prev_pdf[tid] = 0.0f;
+        ps.flags[tid] = 0;
+        ps.split[tid] = NONE;
+    } else {
+        if (ps.terminated[tid]) return;
+        ro = f3m(ps.o[0][tid], ps.o[1][tid], ps.o[2][tid]);
+        rd = f3m(ps.d[0][tid], ps.d[1][tid], ps.d[2][tid]);
+        exclude = ps.exclude[tid];
+    }
+    const float o3[3] = {ro.x, ro.y, ro.z}, d3[3] = {rd.x, rd.y, rd.z};
+    const Hit h = trace_closest(sc, o3, d3, 0.0f, 1e20f, exclude);
+    ps.terminated[tid] = h.prim == NONE ? 1u : 0u;
+    ps.o[0][tid] = h.b1;
+    ps.o[1][tid] = h.b2;
+    ps.o[2][tid] = __uint_as_float(h.prim);
+}
+// the shadow rays of one depth: a light sample that is hidden is taken back
+__global__ void __launch_bounds__(kTraceThreads, 5) k_trace_shadow(SceneView sc, uint32_t n_paths, PathState ps, VertOut v, RecOut rec) {
+    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
+    if (tid >= n_paths || v.dir_pdf[tid] == 0.0f) return;
+    const float o3[3] = {v.ind_wi[0][tid], v.ind_wi[1][tid], v.ind_wi[2][tid]};
+    const float d3[3] = {v.dir_wi[0][tid], v.dir_wi[1][tid], v.dir_wi[2][tid]};
+    const bool hidden = trace_any(sc, o3, d3, 0.0f, v.ind_mis[tid], ps.exclude[tid], ps.light[tid]);
+    v.ind_wi[0][tid] = v.ind_wi[1][tid] = v.ind_wi[2][tid] = 0.0f;
+    v.ind_mis[tid] = 0.0f;
+    if (!hidden) return;
+    v.dir_pdf[tid] = 0.0f;
+    v.dir_wi[0][tid] = v.dir_wi[1][tid] = v.dir_wi[2][tid] = 0.0f;
+    v.dir_l[0][tid] = v.dir_l[1][tid] = v.dir_l[2][tid] = 0.0f;
+    if (rec.rad[0])
+        for (int c = 0; c < 3; c++) rec.rad[c][tid] = v.le[c][tid];
+}
+template <bool SPLIT, bool PRINC, int BLOCKS>
+__global__ void __launch_bounds__(kTraceThreads, BLOCKS) k_trace(SceneView sc, CamArgs cam, uint32_t n_paths, uint32_t depth, uint32_t max_depth,
                         PathState ps, VertOut v, VertOut parent, sty_pcg32 *rng, const sty_style_program *progs,
                         uint32_t n_progs, unsigned long long *vcount, float split_rough, RecOut rec,
                         RecOut rec_parent) {
@@ -59,10 +113,8 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_trace(SceneView sc, CamArg
     float prev_pdf;
     F3 prev_p;
     const bool recs = rec.rad[0] != nullptr;
-    if (depth == 0) {
-        const uint32_t npx = cam.W * cam.H;
-        const uint32_t px = cam.random_px ? pcg_next(st) % npx : cam.pixel_major ? tid / cam.pixel_major : tid % npx;
-        camera_ray(cam, px, st, &ro, &rd);
+    if (!SPLIT && depth == 0) {
+        trace_camera(cam, tid, st, &ro, &rd);
         flags = 0;
         exclude = NONE;
         prev_pdf = 0.0f;
@@ -78,8 +130,15 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_trace(SceneView sc, CamArg
         prev_pdf = ps.prev_pdf[tid];
         prev_p = f3m(ps.prev_p[0][tid], ps.prev_p[1][tid], ps.prev_p[2][tid]);
     }
-    const float o3[3] = {ro.x, ro.y, ro.z}, d3[3] = {rd.x, rd.y, rd.z};
-    const Hit h = trace_closest(sc, o3, d3, 0.0f, 1e20f, exclude);
+    Hit h;
+    if constexpr (SPLIT) {
+        h.b1 = ro.x;
+        h.b2 = ro.y;
+        h.prim = __float_as_uint(ro.z);
+    } else {
+        const float o3[3] = {ro.x, ro.y, ro.z}, d3[3] = {rd.x, rd.y, rd.z};
+        h = trace_closest(sc, o3, d3, 0.0f, 1e20f, exclude);
+    }
     if (h.prim == NONE) {
         ps.terminated[tid] = 1;
         rng[tid] = st;
@@ -143,7 +202,23 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_trace(SceneView sc, CamArg
         F3 lwi;
         f3 li;
         float lpdf;
-        if (nee_sample(sc, p, ng, prim, new_flags, depth, progs, n_progs, st, &lwi, &li, &lpdf)) {
+        bool lit;
+        if constexpr (SPLIT) {  // the shadow ray is k_trace_shadow's
+            NeeSample nee;
+            lit = nee_candidate(sc, p, ng, new_flags, depth, progs, n_progs, st, &nee);
+            if (lit) {
+                lwi = nee.wi;
+                li = nee.li;
+                lpdf = nee.pdf;
+                v.ind_wi[0][tid] = nee.so.x; v.ind_wi[1][tid] = nee.so.y; v.ind_wi[2][tid] = nee.so.z;
+                v.ind_mis[tid] = nee.tmax;
+                ps.light[tid] = nee.lt;
+            }
+            ps.exclude[tid] = prim;
+        } else {
+            lit = nee_sample(sc, p, ng, prim, new_flags, depth, progs, n_progs, st, &lwi, &li, &lpdf);
+        }
+        if (lit) {
             v.dir_wi[0][tid] = lwi.x;
             v.dir_wi[1][tid] = lwi.y;
             v.dir_wi[2][tid] = lwi.z;
@@ -153,7 +228,7 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_trace(SceneView sc, CamArg
             v.dir_pdf[tid] = lpdf;
             if (recs) {  // the direct term of the reference's filter with the vertex as its own neighbour
                 F3 f;
-                const float bp = bsdf_eval(m, ns, ng, wo, lwi, &f, sc.ggx_tab);
+                const float bp = bsdf_eval<PRINC>(m, ns, ng, wo, lwi, &f, sc.ggx_tab);
                 const float w = lpdf / (lpdf + bp) / lpdf;
                 rad = rad + f3m(f.x * li.x, f.y * li.y, f.z * li.z) * w;
                 rec.rad[0][tid] = rad.x; rec.rad[1][tid] = rad.y; rec.rad[2][tid] = rad.z;
@@ -161,7 +236,7 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_trace(SceneView sc, CamArg
         }
     }
     // final-gathering renders stop at the first rough vertex (splitting, nrc_pt.rs:372-375)
-    if (split_rough > 0.0f && lobe_roughness(m, sc.ggx_tab, ns, wo) > split_rough) {
+    if (split_rough > 0.0f && lobe_roughness<PRINC>(m, sc.ggx_tab, ns, wo) > split_rough) {
         ps.split[tid] = depth;
         ps.exclude[tid] = prim;  // the split vertex's triangle, skipped by its gather rays
         ps.terminated[tid] = 1;
@@ -171,10 +246,10 @@ __global__ void __launch_bounds__(kTraceThreads, 6) k_trace(SceneView sc, CamArg
     // BSDF sample and continuation
     const float usel = next_1d(st), us0 = next_1d(st), us1 = next_1d(st);
     float pdf = 0.0f;
-    const F3 wi = bsdf_sample(m, ns, ng, wo, usel, us0, us1, &pdf, sc.ggx_tab);
+    const F3 wi = bsdf_sample<PRINC>(m, ns, ng, wo, usel, us0, us1, &pdf, sc.ggx_tab);
     if (recs && pdf > 0.0f) {  // throughput to the child: f |cos| / pdf (times the child's MIS weight, above)
         F3 f;
-        const float bp = bsdf_eval(m, ns, ng, wo, wi, &f, sc.ggx_tab);
+        const float bp = bsdf_eval<PRINC>(m, ns, ng, wo, wi, &f, sc.ggx_tab);
         if (bp > 0.0f) {
             const float k = 1.0f / bp;
             rec.thr[0][tid] = f.x * k; rec.thr[1][tid] = f.y * k; rec.thr[2][tid] = f.z * k;
@@ -416,43 +491,14 @@ __global__ void k_split_collect(uint32_t n, uint32_t d, VertOut v, const uint32_
 // One gather iteration for every split path: another light sample at the split vertex (added to
 // acc_direct) and one BSDF-sampled ray; its hit becomes a cache query row (zero row if none) with
 // the sample's throughput f |cos| / pdf and the hit's emission MIS weight.
-__global__ void k_fg_step(SceneView sc, FeatArgs fa, uint32_t n, const uint32_t *split, SplitPlanes sp, sty_pcg32 *rng,
-                          const sty_style_program *progs, uint32_t n_progs, float *rows, float *thr, float *gmis,
-                          uint32_t *gmat, uint32_t *gflags, float *gpos, float *acc_direct) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float *row = rows + (size_t)i * fa.dims;
-    for (uint32_t c = 0; c < fa.dims; c++) row[c] = 0.0f;
-    thr[i] = thr[n + i] = thr[2 * (size_t)n + i] = 0.0f;
-    const uint32_t s = split[i];
-    if (s == NONE) return;
-    sty_pcg32 st = rng[i];
-    const sty_scene_material m = sc.materials[sp.material[i]];
-    const F3 p = f3m(sp.p[0][i], sp.p[1][i], sp.p[2][i]), wo = f3m(sp.wo[0][i], sp.wo[1][i], sp.wo[2][i]);
-    const F3 ns = f3m(sp.ns[0][i], sp.ns[1][i], sp.ns[2][i]), ng = f3m(sp.ng[0][i], sp.ng[1][i], sp.ng[2][i]);
-    const uint32_t fl = sp.flags[i], prim = sp.prim[i];
-    {
-        F3 lwi;
-        f3 li;
-        float lpdf;
-        if (nee_sample(sc, p, ng, prim, fl, s, progs, n_progs, st, &lwi, &li, &lpdf)) {
-            F3 f;
-            const float bp = bsdf_eval(m, ns, ng, wo, lwi, &f, sc.ggx_tab);
-            const float w = lpdf / (lpdf + bp) / lpdf;
-            acc_direct[i] += f.x * li.x * w;
-            acc_direct[n + i] += f.y * li.y * w;
-            acc_direct[2 * (size_t)n + i] += f.z * li.z * w;
-        }
-    }
-    const float usel = next_1d(st), us0 = next_1d(st), us1 = next_1d(st);
-    float pdf = 0.0f;
-    const F3 wi = bsdf_sample(m, ns, ng, wo, usel, us0, us1, &pdf, sc.ggx_tab);
-    rng[i] = st;
-    if (!(pdf > 0.0f)) return;
-    const F3 o = offset_ray_origin(p, face_forward(ng, wi));
-    const float o3[3] = {o.x, o.y, o.z}, d3[3] = {wi.x, wi.y, wi.z};
-    const Hit h = trace_closest(sc, o3, d3, 0.0f, 1e20f, prim);
-    if (h.prim == NONE) return;
+// what a gather ray that left the split vertex p along wi brings back from its hit
+struct GatherOut {
+    float *rows, *thr, *gmis;
+    uint32_t *gmat, *gflags;
+    float *gpos;
+};
+__device__ __forceinline__ float gather_hit(const SceneView &sc, const Hit &h, F3 p, float pdf, uint32_t fl, F3 *q_out, F3 *qn_out,
+                                            uint32_t *qm_out, uint32_t *qf_out) {
     const float *tp = sc.tri_pos + 9 * (size_t)h.prim;
     const float b0 = 1.0f - h.b1 - h.b2;
     const F3 q = f3m(b0 * tp[0] + h.b1 * tp[3] + h.b2 * tp[6], b0 * tp[1] + h.b1 * tp[4] + h.b2 * tp[7],
@@ -477,19 +523,148 @@ __global__ void k_fg_step(SceneView sc, FeatArgs fa, uint32_t n, const uint32_t 
         if (mq.set_style == 2) qf |= 4u;
         if (mq.set_style == 3) qf |= 8u;
     }
+    *q_out = q;
+    *qn_out = qn;
+    *qm_out = qm;
+    *qf_out = qf;
+    return mis;
+}
+__device__ __forceinline__ void gather_write(const SceneView &sc, const FeatArgs &fa, uint32_t n, uint32_t i, uint32_t s, F3 wi, F3 q, F3 qn,
+                                             uint32_t qm, uint32_t qf, float mis, const GatherOut &g) {
+    g.gmis[i] = mis;
+    g.gmat[i] = qm;
+    g.gflags[i] = qf;
+    g.gpos[i] = q.x;
+    g.gpos[n + i] = q.y;
+    g.gpos[2 * (size_t)n + i] = q.z;
+    write_features(sc, fa, q, -wi, qn, qm, qf, s + 1, g.rows + (size_t)i * fa.dims);
+}
+// Scenes with closures: the samples (k_fg_step<true>), their rays (k_fg_walk) and what they bring (k_fg_hit) apart, as in
+// k_trace and for its reason (16 gather rays per pixel, principled Cornell box at 768 x 768: a frame of 8.7 ms; in one
+// kernel 9.0 on the binary tree, 15.0 on the wide one). The path's planes, free after the trace, carry them: shadow ray prev_p, gpos (direction),
+// flags (length), light (its triangle; NONE: no ray, or hidden), the sample it carries in the row's first
+// columns with its weight in `terminated`; gather ray o, d, prev_pdf (0: none), after the walk o = barycentrics, triangle.
+template <bool SPLIT>
+__global__ void k_fg_step(SceneView sc, FeatArgs fa, uint32_t n, const uint32_t *split, SplitPlanes sp, PathState ps, sty_pcg32 *rng,
+                          const sty_style_program *progs, uint32_t n_progs, GatherOut g, float *acc_direct) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    float *const row = g.rows + (size_t)i * fa.dims, *const thr = g.thr;
+    for (uint32_t c = 0; c < fa.dims; c++) row[c] = 0.0f;
+    thr[i] = thr[n + i] = thr[2 * (size_t)n + i] = 0.0f;
+    const uint32_t s = split[i];
+    if (SPLIT) {
+        ps.light[i] = NONE;
+        ps.prev_pdf[i] = 0.0f;
+    }
+    if (s == NONE) return;
+    sty_pcg32 st = rng[i];
+    const sty_scene_material m = sc.materials[sp.material[i]];
+    const F3 p = f3m(sp.p[0][i], sp.p[1][i], sp.p[2][i]), wo = f3m(sp.wo[0][i], sp.wo[1][i], sp.wo[2][i]);
+    const F3 ns = f3m(sp.ns[0][i], sp.ns[1][i], sp.ns[2][i]), ng = f3m(sp.ng[0][i], sp.ng[1][i], sp.ng[2][i]);
+    const uint32_t fl = sp.flags[i], prim = sp.prim[i];
+    if constexpr (SPLIT) {
+        NeeSample nee;
+        if (nee_candidate(sc, p, ng, fl, s, progs, n_progs, st, &nee)) {
+            F3 f;
+            const float bp = bsdf_eval<SPLIT>(m, ns, ng, wo, nee.wi, &f, sc.ggx_tab);
+            const float w = nee.pdf / (nee.pdf + bp) / nee.pdf;
+            row[0] = f.x * nee.li.x;
+            row[1] = f.y * nee.li.y;
+            row[2] = f.z * nee.li.z;
+            ps.terminated[i] = __float_as_uint(w);
+            ps.prev_p[0][i] = nee.so.x; ps.prev_p[1][i] = nee.so.y; ps.prev_p[2][i] = nee.so.z;
+            g.gpos[i] = nee.wi.x; g.gpos[n + i] = nee.wi.y; g.gpos[2 * (size_t)n + i] = nee.wi.z;
+            ps.flags[i] = __float_as_uint(nee.tmax);
+            ps.light[i] = nee.lt;
+        }
+    } else {
+        F3 lwi;
+        f3 li;
+        float lpdf;
+        if (nee_sample(sc, p, ng, prim, fl, s, progs, n_progs, st, &lwi, &li, &lpdf)) {
+            F3 f;
+            const float bp = bsdf_eval<SPLIT>(m, ns, ng, wo, lwi, &f, sc.ggx_tab);
+            const float w = lpdf / (lpdf + bp) / lpdf;
+            acc_direct[i] += f.x * li.x * w;
+            acc_direct[n + i] += f.y * li.y * w;
+            acc_direct[2 * (size_t)n + i] += f.z * li.z * w;
+        }
+    }
+    const float usel = next_1d(st), us0 = next_1d(st), us1 = next_1d(st);
+    float pdf = 0.0f;
+    const F3 wi = bsdf_sample<SPLIT>(m, ns, ng, wo, usel, us0, us1, &pdf, sc.ggx_tab);
+    rng[i] = st;
+    if (!(pdf > 0.0f)) return;
+    const F3 o = offset_ray_origin(p, face_forward(ng, wi));
     F3 f;
-    const float bp = bsdf_eval(m, ns, ng, wo, wi, &f, sc.ggx_tab);
-    if (!(bp > 0.0f)) return;
-    thr[i] = f.x / bp;
-    thr[n + i] = f.y / bp;
-    thr[2 * (size_t)n + i] = f.z / bp;
-    gmis[i] = mis;
-    gmat[i] = qm;
-    gflags[i] = qf;
-    gpos[i] = q.x;
-    gpos[n + i] = q.y;
-    gpos[2 * (size_t)n + i] = q.z;
-    write_features(sc, fa, q, -wi, qn, qm, qf, s + 1, row);
+    if constexpr (SPLIT) {
+        const float bp = bsdf_eval<SPLIT>(m, ns, ng, wo, wi, &f, sc.ggx_tab);
+        if (!(bp > 0.0f)) return;
+        thr[i] = f.x / bp;
+        thr[n + i] = f.y / bp;
+        thr[2 * (size_t)n + i] = f.z / bp;
+        ps.o[0][i] = o.x; ps.o[1][i] = o.y; ps.o[2][i] = o.z;
+        ps.d[0][i] = wi.x; ps.d[1][i] = wi.y; ps.d[2][i] = wi.z;
+        ps.prev_pdf[i] = pdf;
+    } else {
+        const float o3[3] = {o.x, o.y, o.z}, d3[3] = {wi.x, wi.y, wi.z};
+        const Hit h = trace_closest(sc, o3, d3, 0.0f, 1e20f, prim);
+        if (h.prim == NONE) return;
+        F3 q, qn;
+        uint32_t qm, qf;
+        const float mis = gather_hit(sc, h, p, pdf, fl, &q, &qn, &qm, &qf);
+        const float bp = bsdf_eval<SPLIT>(m, ns, ng, wo, wi, &f, sc.ggx_tab);
+        if (!(bp > 0.0f)) return;
+        thr[i] = f.x / bp;
+        thr[n + i] = f.y / bp;
+        thr[2 * (size_t)n + i] = f.z / bp;
+        gather_write(sc, fa, n, i, s, wi, q, qn, qm, qf, mis, g);
+    }
+}
+__global__ void __launch_bounds__(kTraceThreads, 5) k_fg_walk(SceneView sc, uint32_t n, SplitPlanes sp, PathState ps, const float *gpos) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, i = t < n ? t : t - n;
+    if (i >= n) return;
+    if (t < n) {
+        const uint32_t lt = ps.light[i];
+        if (lt == NONE) return;
+        const float o3[3] = {ps.prev_p[0][i], ps.prev_p[1][i], ps.prev_p[2][i]}, d3[3] = {gpos[i], gpos[n + i], gpos[2 * (size_t)n + i]};
+        if (trace_any(sc, o3, d3, 0.0f, __uint_as_float(ps.flags[i]), sp.prim[i], lt)) ps.light[i] = NONE;
+    } else {
+        if (ps.prev_pdf[i] == 0.0f) return;
+        const float o3[3] = {ps.o[0][i], ps.o[1][i], ps.o[2][i]}, d3[3] = {ps.d[0][i], ps.d[1][i], ps.d[2][i]};
+        const Hit h = trace_closest(sc, o3, d3, 0.0f, 1e20f, sp.prim[i]);
+        ps.o[0][i] = h.b1;
+        ps.o[1][i] = h.b2;
+        ps.o[2][i] = __uint_as_float(h.prim);
+    }
+}
+__global__ void __launch_bounds__(kTraceThreads) k_fg_hit(SceneView sc, FeatArgs fa, uint32_t n, const uint32_t *split, SplitPlanes sp, PathState ps,
+                                                          GatherOut g, float *acc_direct) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t s = split[i];
+    if (s == NONE) return;
+    float *row = g.rows + (size_t)i * fa.dims;
+    if (ps.light[i] != NONE) {
+        const float w = __uint_as_float(ps.terminated[i]);
+        for (int c = 0; c < 3; c++) acc_direct[c * (size_t)n + i] = __fmaf_rn(row[c], w, acc_direct[c * (size_t)n + i]);
+    }
+    row[0] = row[1] = row[2] = 0.0f;
+    const float pdf = ps.prev_pdf[i];
+    if (pdf == 0.0f) return;
+    Hit h;
+    h.b1 = ps.o[0][i];
+    h.b2 = ps.o[1][i];
+    h.prim = __float_as_uint(ps.o[2][i]);
+    if (h.prim == NONE) {
+        g.thr[i] = g.thr[n + i] = g.thr[2 * (size_t)n + i] = 0.0f;
+        return;
+    }
+    F3 q, qn;
+    uint32_t qm, qf;
+    const float mis = gather_hit(sc, h, f3m(sp.p[0][i], sp.p[1][i], sp.p[2][i]), pdf, sp.flags[i], &q, &qn, &qm, &qf);
+    gather_write(sc, fa, n, i, s, f3m(ps.d[0][i], ps.d[1][i], ps.d[2][i]), q, qn, qm, qf, mis, g);
 }
 // acc_indirect += style_{s+1}(cache prediction at the gather hit) * throughput * mis; every
 // iteration counts (a miss contributes 0)
@@ -661,7 +836,7 @@ struct TraceJob {
         scene_bounds(scene, bmin, bmax);
         verts = (float *)alloc(kVerts, (size_t)D * kPlanes * n * 4, "alloc vertices");
         outs = (float *)alloc(kOuts, (size_t)D * 3 * n * 4, "alloc outputs");
-        psb = (float *)alloc(kPathState, (size_t)14 * n * 4, "alloc path state");
+        psb = (float *)alloc(kPathState, (size_t)15 * n * 4, "alloc path state");
         rng = (sty_pcg32 *)alloc(kRng, (size_t)n * sizeof(sty_pcg32), "alloc rng");
         dprog = (sty_style_program *)alloc(kPrograms, 64 * sizeof(sty_style_program), "alloc programs");
         vc = (unsigned long long *)alloc(kVertexCount, 8, "alloc counter");
@@ -720,6 +895,7 @@ struct TraceJob {
         ps.exclude = (uint32_t *)pl();
         ps.terminated = (uint32_t *)pl();
         ps.split = (uint32_t *)pl();
+        ps.light = (uint32_t *)pl();
         ro.assign(D, RecOut{});
         k_rng_init<<<(n + 255) / 256, 256, 0, st>>>(n, std_rng_key_of(seed), pixel_major, npx, rng);
         return check_launch("k_rng_init");
@@ -788,11 +964,30 @@ struct TraceJob {
             STY_TRY(check_cuda(cudaMemsetAsync(rp.valid, 0, pl, st), "reset records"));
             if (rp.prim) STY_TRY(check_cuda(cudaMemsetAsync(rp.prim, 0xff, pl, st), "reset records"));
         }
+        int dev = 0, sms = 0;
+        STY_TRY(check_cuda(cudaGetDevice(&dev), "cudaGetDevice"));
+        STY_TRY(check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr SMs"));
+        const unsigned blocks = (n + kTraceThreads - 1) / kTraceThreads, per_sm = (blocks + (unsigned)sms - 1) / (unsigned)sms;
+        // Blocks per SM: 2 (no spills) where there are no more than that, 4 up to 8, else 5. Cornell box, 2 / 4 / 5 / 6 of
+        // them: 65 k paths 0.364 / 0.368 / 0.384 / 0.398 ms, 147 k 0.540 / 0.510 / 0.524 / 0.548, 3.1 M 6.53 / 5.63 / 5.68 /
+        // 5.78; room, 3.1 M 19.9 / 15.3 / 15.0 / 15.1. Three kernels for closures from the second block per SM on:
+        // 65 k paths 0.55 ms, 0.68 in one kernel; 16 k 0.48 and 0.44.
+        const bool princ = sv.any_closure != 0, split = princ && per_sm > 1;
+        const auto kernel = split ? k_trace<true, true, 2> : princ ? k_trace<false, true, 2>
+                            : per_sm > 8 ? k_trace<false, false, 5> : per_sm > 2 ? k_trace<false, false, 4> : k_trace<false, false, 2>;
         for (uint32_t d = 0; d < D; d++) {
-            k_trace<<<(n + kTraceThreads - 1) / kTraceThreads, kTraceThreads, 0, st>>>(sv, ca, n, d, max_depth, ps, vo[d], vo[d > 0 ? d - 1 : 0], rng,
-                                                     dprog, n_programs, vc, split_rough, ro[d],
-                                                     ro[d > 0 ? d - 1 : 0]);
+            if (split) {
+                k_trace_hits<<<blocks, kTraceThreads, 0, st>>>(sv, ca, n, d, ps, rng);
+                STY_TRY(check_launch("k_trace_hits"));
+            }
+            kernel<<<blocks, kTraceThreads, 0, st>>>(
+                sv, ca, n, d, max_depth, ps, vo[d], vo[d > 0 ? d - 1 : 0], rng, dprog, n_programs, vc, split_rough, ro[d],
+                ro[d > 0 ? d - 1 : 0]);
             STY_TRY(check_launch("k_trace"));
+            if (split && d < max_depth) {
+                k_trace_shadow<<<blocks, kTraceThreads, 0, st>>>(sv, n, ps, vo[d], ro[d]);
+                STY_TRY(check_launch("k_trace_shadow"));
+            }
         }
         return STY_OK;
     }
@@ -1247,10 +1442,18 @@ extern "C" sty_status sty_nrc_render(sty_scene *scene, sty_nrc *nrc, const sty_n
             k_split_collect<<<nb, 256, 0, st>>>(npx, d, job.vo[d], job.ps.split, job.ps.exclude, sp);
             STY_TRY(check_launch("k_split_collect"));
         }
+        const GatherOut gout = {qin, thr, gmis, gmat, gflags, gpos};
+        const bool closures = job.sv.any_closure != 0;
         for (uint32_t it = 0; it < fg; it++) {
-            k_fg_step<<<nb, 256, 0, st>>>(job.sv, fa, npx, job.ps.split, sp, job.rng, job.dprog, n_programs, qin, thr, gmis,
-                                          gmat, gflags, gpos, acc_direct);
+            (closures ? k_fg_step<true> : k_fg_step<false>)<<<nb, 256, 0, st>>>(job.sv, fa, npx, job.ps.split, sp, job.ps, job.rng,
+                                                                                job.dprog, n_programs, gout, acc_direct);
             STY_TRY(check_launch("k_fg_step"));
+            if (closures) {
+                k_fg_walk<<<(unsigned)((2 * (uint64_t)npx + 255) / 256), 256, 0, st>>>(job.sv, npx, sp, job.ps, gpos);
+                STY_TRY(check_launch("k_fg_walk"));
+                k_fg_hit<<<nb, 256, 0, st>>>(job.sv, fa, npx, job.ps.split, sp, job.ps, gout, acc_direct);
+                STY_TRY(check_launch("k_fg_hit"));
+            }
             STY_TRY(sty_nrc_inference(nrc, npx, qin, qpred, stream));
             acc.inference_queries += npx;
             k_fg_accumulate<<<nb, 256, 0, st>>>(job.sv, npx, job.ps.split, qpred, thr, gmis, gmat, gflags, gpos,

@@ -195,6 +195,7 @@ struct PathState {
     float *prev_pdf;
     uint32_t *flags, *exclude, *terminated;
     uint32_t *split;  // depth of the vertex a final-gathering render stopped at, NONE otherwise
+    uint32_t *light;  // the light sample's triangle, between the kernels of a depth that has several (trace.cu)
 };
 struct VertOut {  // mutable view of one depth's sty_pf_vertices planes
     int32_t *active;
