@@ -148,13 +148,16 @@ struct RayBox {
 };
 __device__ __forceinline__ RayBox ray_box(const float o[3], const float d[3]) {
     RayBox r;
+    // A direction component of (nearly) 0 beside the others as 1e-24 of the largest: finite, so that the axis still excludes
+    // the boxes the ray passes; the boxes' margin keeps those it lies in or touches. Where that underflows (directions
+    // below 1e-14) the inverse is infinite, every plane's distance a NaN, and the axis excludes nothing.
+    const float least = 1e-24f * fmaxf(fmaxf(fabsf(d[0]), fabsf(d[1])), fabsf(d[2]));
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         r.o[a] = o[a];
-        // a direction component of (nearly) 0 as +-1e-24: finite, so that the axis still excludes the boxes the
-        // ray passes; the boxes' margin keeps those it lies in or touches
-        // (an approximate reciprocal: its error scales both planes alike, far below the widening)
-        r.inv[a] = __fdividef(1.0f, fabsf(d[a]) < 1e-24f ? copysignf(1e-24f, d[a]) : d[a]);
+        const float v = fabsf(d[a]) < least ? copysignf(least, d[a]) : d[a];
+        // (an approximate reciprocal: its error scales both planes alike, far below the widening; it is 0 past 2^126)
+        r.inv[a] = fabsf(v) > 0x1p125f ? 1.0f / v : __fdividef(1.0f, v);
     }
     return r;
 }
