@@ -41,25 +41,25 @@ struct AdjArgs {
 
 __device__ __forceinline__ float sigm(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-// What a query holds during the sweep. The exponent is formed negated, -a log2(e) = om' + d2 isp' + rho isx' with
-// om' = isn' (1 - n_i.n_j) summed from the candidate's bias, isn' where the record is valid and kNone where it
-// is not: its weight is then exactly 0.
-constexpr float kNone = 1e30f;
+// What a query holds during the sweep. The exponent is formed negated, -a log2(e) = isn' om + isp' d2 + isx' rho with
+// om = 1 - n_i.n_j summed from the candidate's bias, 1 where the record is valid and kNone where it is not: its weight is
+// then exactly 0, for which isn' is kept from falling below kLeast (where om has no weight left any more).
+constexpr float kNone = 1e30f, kLeast = 1e-20f;
 struct Query {
-    float p[3], n[3];   // position; normal times -isn'
+    float p[3], n[3];   // position; normal, negated
     float h[3], nhf;    // dL/df; -h.f
 };
 struct Sums {
-    float d, e[3];  // sum w; sums of t = w h.(in_j - f_i) times rho, d2, om'
+    float d, e[3];  // sum w; sums of t = w h.(in_j - f_i) times rho, d2, om
 };
 
 // One candidate row for 4 spp on packed FP32: a candidate pixel's 4 samples come in as one 16-byte load per
 // field and are paired (0, 1) and (2, 3) against a query duplicated in both lanes, so no value has to be
 // moved into a pair. 19 FFMA2 and 2 MUFU per query and pair.
 __device__ __forceinline__ void row4(const float *__restrict__ rowp, int plane, int lx, int R, int dy, float isx2, float isp2,
-                                     const Query (&q)[4], Sums (&out)[4]) {
+                                     float isn, const Query (&q)[4], Sums (&out)[4]) {
     const float2 zero2 = make_float2(0.0f, 0.0f), one2 = make_float2(1.0f, 1.0f), m1 = make_float2(-1.0f, -1.0f);
-    const float2 isp = make_float2(isp2, isp2);
+    const float2 isp = make_float2(isp2, isp2), isn2 = make_float2(isn, isn);
     float2 acc[4][4];
 #pragma unroll
     for (int k = 0; k < 4; k++)
@@ -85,7 +85,7 @@ __device__ __forceinline__ void row4(const float *__restrict__ rowp, int plane, 
                              ez = ffma2(c[2], m1, two(q[k].p[2]));
                 const float2 d2 = ffma2(ez, ez, ffma2(ey, ey, ffma2(ex, ex, zero2)));
                 const float2 om = ffma2(two(q[k].n[2]), c[5], ffma2(two(q[k].n[1]), c[4], ffma2(two(q[k].n[0]), c[3], c[6])));
-                const float2 na = ffma2(ffma2(d2, isp, om), one2, arho);
+                const float2 na = ffma2(om, isn2, ffma2(d2, isp, arho));
                 const float2 w = make_float2(ex2_approx(-na.x), ex2_approx(-na.y));
                 const float2 u = ffma2(two(q[k].h[2]), c[9], ffma2(two(q[k].h[1]), c[8], ffma2(two(q[k].h[0]), c[7], two(q[k].nhf))));
                 const float2 tt = ffma2(w, u, zero2);
@@ -105,7 +105,7 @@ __device__ __forceinline__ void row4(const float *__restrict__ rowp, int plane, 
 }
 template <int S>
 __device__ __forceinline__ void row_any(const float *__restrict__ rowp, int plane, int lx, int R, int dy, float isx2, float isp2,
-                                        const Query (&q)[S], Sums (&out)[S]) {
+                                        float isn, const Query (&q)[S], Sums (&out)[S]) {
 #pragma unroll
     for (int k = 0; k < S; k++) out[k] = {0.0f, {0.0f, 0.0f, 0.0f}};
     for (int dx = -R; dx <= R; dx++) {
@@ -121,7 +121,7 @@ __device__ __forceinline__ void row_any(const float *__restrict__ rowp, int plan
                 const float ex = q[k].p[0] - c[0], ey = q[k].p[1] - c[1], ez = q[k].p[2] - c[2];
                 const float d2 = ex * ex + ey * ey + ez * ez;
                 const float om = fmaf(q[k].n[2], c[5], fmaf(q[k].n[1], c[4], fmaf(q[k].n[0], c[3], c[6])));
-                const float w = ex2_approx(-(fmaf(d2, isp2, om) + rho * isx2));
+                const float w = ex2_approx(-fmaf(om, isn, fmaf(d2, isp2, rho * isx2)));
                 const float tt = w * fmaf(q[k].h[2], c[9], fmaf(q[k].h[1], c[8], fmaf(q[k].h[0], c[7], q[k].nhf)));
                 out[k].d += w;
                 out[k].e[0] = fmaf(tt, rho, out[k].e[0]);
@@ -148,7 +148,8 @@ __global__ void __launch_bounds__(NT, S == 4 ? 3 : 1) k_pf_adjoint(const AdjArgs
     const int x = tx0 + lx, y = ty0 + ly;
     const bool inside = x < a.W && y < a.H;
     const size_t N = (size_t)a.W * a.H * S, dbase = (size_t)a.depth * N;
-    const float isx2 = kL2E / (2.0f * a.sx * a.sx), isp2 = kL2E / (2.0f * a.sp * a.sp), isn = kL2E / (a.sn * a.sn);
+    const float isx2 = kL2E / (2.0f * a.sx * a.sx), isp2 = kL2E / (2.0f * a.sp * a.sp),
+                isn = fmaxf(kL2E / (a.sn * a.sn), kLeast);
 
     // a warp's sums of gradient entries k0 .. k0 + n - 1
     auto reduce = [&](const float *v0, int k0, int n) {
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(NT, S == 4 ? 3 : 1) k_pf_adjoint(const AdjArgs
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             q[s].p[k] = inside ? a.pos[k][g] : 0.0f;
-            q[s].n[k] = inside ? a.nrm[k][g] * -isn : 0.0f;
+            q[s].n[k] = inside ? -a.nrm[k][g] : 0.0f;
             q[s].h[k] = 0.0f;
         }
         if (!qv[s]) continue;
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(NT, S == 4 ? 3 : 1) k_pf_adjoint(const AdjArgs
                 }
                 sm[(7 + k) * plane + idx] = in;
             }
-            sm[6 * plane + idx] = ok ? isn : kNone;
+            sm[6 * plane + idx] = ok ? 1.0f : kNone;
         }
         __syncthreads();
         for (int r = 0; r < CH; r++) {
@@ -248,8 +249,8 @@ __global__ void __launch_bounds__(NT, S == 4 ? 3 : 1) k_pf_adjoint(const AdjArgs
             if (dy < -R || dy > R) continue;
             Sums part[S];
             const float *rowp = sm + r * CW * S;
-            if constexpr (S == 4) row4(rowp, plane, lx, R, dy, isx2, isp2, q, part);
-            else row_any<S>(rowp, plane, lx, R, dy, isx2, isp2, q, part);
+            if constexpr (S == 4) row4(rowp, plane, lx, R, dy, isx2, isp2, isn, q, part);
+            else row_any<S>(rowp, plane, lx, R, dy, isx2, isp2, isn, q, part);
 #pragma unroll
             for (int s = 0; s < S; s++) {
                 acc[s][0].add(part[s].d);
@@ -265,7 +266,7 @@ __global__ void __launch_bounds__(NT, S == 4 ? 3 : 1) k_pf_adjoint(const AdjArgs
         const float inv = 1.0f / acc[s][0].s;
         bw[0] += acc[s][1].s * inv / (a.sx * a.sx * a.sx);
         bw[1] += acc[s][2].s * inv / (a.sp * a.sp * a.sp);
-        bw[2] += 2.0f * (acc[s][3].s / isn) * inv / (a.sn * a.sn * a.sn);
+        bw[2] += 2.0f * acc[s][3].s * inv / (a.sn * a.sn * a.sn);
     }
     reduce(bw, NG - 3, 3);
     __syncthreads();
