@@ -9,9 +9,10 @@
 //           with Y the Rec.709 luminance weights;
 //   filter: df_i/dtheta = sum_j dw_ij/dtheta (in_j - f_i) / D_i with dw/dsx = w rho / sx^3,
 //           dw/dsp = w |dp|^2 / sp^3, dw/dsn = 2 w (1 - n.n) / sn^3.
-// f_i comes from the forward filter, so one sweep over the staged candidate rows accumulates D_i and the
-// three bandwidth sums. Per-thread results are reduced per block into a partial vector; one block per entry
-// sums the partials in a fixed order (deterministic).
+// The image and its loss are the forward filter's. The sweep over the staged candidate rows sums D_i and the three bandwidth
+// terms with f_i and h_i; where sweep_gives_f() a sweep of the same kernel before it has formed f_i by the same
+// operations. Per-thread results are reduced per block into a partial vector; one block per entry sums the partials in a
+// fixed order (deterministic).
 #include <mutex>
 
 #include "common.cuh"
@@ -30,7 +31,7 @@ struct AdjArgs {
     const int32_t *valid;
     const float *in_next;
     const float *dimg;  // dL/dimage per pixel, interleaved rgb
-    const float *f;     // filtered radiance, planes of W H S
+    float *f;           // filtered radiance, planes of W H S
     int W, H, R;
     uint32_t depth;
     float sx, sp, sn;
@@ -50,12 +51,13 @@ struct Query {
     float h[3], nhf;    // dL/df; -h.f
 };
 struct Sums {
-    float d, e[3];  // sum w; sums of t = w h.(in_j - f_i) times rho, d2, om
+    float d, e[3];  // sum w; first sweep: sums of w in; second: sums of t = w h.(in_j - f_i) times rho, d2, om
 };
 
 // One candidate row for 4 spp on packed FP32: a candidate pixel's 4 samples come in as one 16-byte load per
 // field and are paired (0, 1) and (2, 3) against a query duplicated in both lanes, so no value has to be
-// moved into a pair. 19 FFMA2 and 2 MUFU per query and pair.
+// moved into a pair. 15 (first sweep) or 19 FFMA2 and 2 MUFU per query and pair.
+template <bool FIRST>
 __device__ __forceinline__ void row4(const float *__restrict__ rowp, int plane, int lx, int R, int dy, float isx2, float isp2,
                                      float isn, const Query (&q)[4], Sums (&out)[4]) {
     const float2 zero2 = make_float2(0.0f, 0.0f), one2 = make_float2(1.0f, 1.0f), m1 = make_float2(-1.0f, -1.0f);
@@ -87,12 +89,17 @@ __device__ __forceinline__ void row4(const float *__restrict__ rowp, int plane, 
                 const float2 om = ffma2(two(q[k].n[2]), c[5], ffma2(two(q[k].n[1]), c[4], ffma2(two(q[k].n[0]), c[3], c[6])));
                 const float2 na = ffma2(om, isn2, ffma2(d2, isp, arho));
                 const float2 w = make_float2(ex2_approx(-na.x), ex2_approx(-na.y));
-                const float2 u = ffma2(two(q[k].h[2]), c[9], ffma2(two(q[k].h[1]), c[8], ffma2(two(q[k].h[0]), c[7], two(q[k].nhf))));
-                const float2 tt = ffma2(w, u, zero2);
                 acc[k][0] = ffma2(w, one2, acc[k][0]);
-                acc[k][1] = ffma2(tt, rho2, acc[k][1]);
-                acc[k][2] = ffma2(tt, d2, acc[k][2]);
-                acc[k][3] = ffma2(tt, om, acc[k][3]);
+                if constexpr (FIRST) {
+#pragma unroll
+                    for (int j = 0; j < 3; j++) acc[k][1 + j] = ffma2(w, c[7 + j], acc[k][1 + j]);
+                } else {
+                    const float2 u = ffma2(two(q[k].h[2]), c[9], ffma2(two(q[k].h[1]), c[8], ffma2(two(q[k].h[0]), c[7], two(q[k].nhf))));
+                    const float2 tt = ffma2(w, u, zero2);
+                    acc[k][1] = ffma2(tt, rho2, acc[k][1]);
+                    acc[k][2] = ffma2(tt, d2, acc[k][2]);
+                    acc[k][3] = ffma2(tt, om, acc[k][3]);
+                }
             }
         }
     }
@@ -103,13 +110,13 @@ __device__ __forceinline__ void row4(const float *__restrict__ rowp, int plane, 
         for (int j = 0; j < 3; j++) out[k].e[j] = acc[k][j + 1].x + acc[k][j + 1].y;
     }
 }
-template <int S>
+template <int S, bool FIRST>
 __device__ __forceinline__ void row_any(const float *__restrict__ rowp, int plane, int lx, int R, int dy, float isx2, float isp2,
                                         float isn, const Query (&q)[S], Sums (&out)[S]) {
 #pragma unroll
     for (int k = 0; k < S; k++) out[k] = {0.0f, {0.0f, 0.0f, 0.0f}};
     for (int dx = -R; dx <= R; dx++) {
-        const float rho = (float)(dx * dx + dy * dy);
+        const float rho = (float)(dx * dx + dy * dy), arho = __fmul_rn(rho, isx2);
         const int cb = (lx + R + dx) * S;
 #pragma unroll
         for (int t = 0; t < S; t++) {
@@ -119,14 +126,19 @@ __device__ __forceinline__ void row_any(const float *__restrict__ rowp, int plan
 #pragma unroll
             for (int k = 0; k < S; k++) {
                 const float ex = q[k].p[0] - c[0], ey = q[k].p[1] - c[1], ez = q[k].p[2] - c[2];
-                const float d2 = ex * ex + ey * ey + ez * ez;
+                const float d2 = fmaf(ez, ez, fmaf(ey, ey, __fmul_rn(ex, ex)));
                 const float om = fmaf(q[k].n[2], c[5], fmaf(q[k].n[1], c[4], fmaf(q[k].n[0], c[3], c[6])));
-                const float w = ex2_approx(-fmaf(om, isn, fmaf(d2, isp2, rho * isx2)));
-                const float tt = w * fmaf(q[k].h[2], c[9], fmaf(q[k].h[1], c[8], fmaf(q[k].h[0], c[7], q[k].nhf)));
+                const float w = ex2_approx(-fmaf(om, isn, fmaf(d2, isp2, arho)));
                 out[k].d += w;
-                out[k].e[0] = fmaf(tt, rho, out[k].e[0]);
-                out[k].e[1] = fmaf(tt, d2, out[k].e[1]);
-                out[k].e[2] = fmaf(tt, om, out[k].e[2]);
+                if constexpr (FIRST) {
+#pragma unroll
+                    for (int j = 0; j < 3; j++) out[k].e[j] = fmaf(w, c[7 + j], out[k].e[j]);
+                } else {
+                    const float tt = w * fmaf(q[k].h[2], c[9], fmaf(q[k].h[1], c[8], fmaf(q[k].h[0], c[7], q[k].nhf)));
+                    out[k].e[0] = fmaf(tt, rho, out[k].e[0]);
+                    out[k].e[1] = fmaf(tt, d2, out[k].e[1]);
+                    out[k].e[2] = fmaf(tt, om, out[k].e[2]);
+                }
             }
         }
     }
@@ -137,7 +149,7 @@ __device__ __forceinline__ void row_any(const float *__restrict__ rowp, int plan
 // sweeps (the first for f and D), a candidate duplicated into each pair, 220 registers and one block of
 // 8 warps per SM; 1.88 with one sweep on the forward filter's f, 1.66 with blocks of 32 x 4 pixels, three
 // to an SM (32 x 12, one to an SM: 1.81).
-template <int S>
+template <int S, bool FIRST>
 __global__ void __launch_bounds__(NT, S == 4 ? 3 : 1) k_pf_adjoint(const AdjArgs a) {
     extern __shared__ __align__(16) float sm[];
     __shared__ float red[NT / 32][NG];
@@ -163,7 +175,7 @@ __global__ void __launch_bounds__(NT, S == 4 ? 3 : 1) k_pf_adjoint(const AdjArgs
     };
     Query q[S];
     bool qv[S];
-    // queries; style backward from the forward filter's f
+    // queries; in the second sweep the style's backward from f
     {
     float gsum[NG - 3];
 #pragma unroll
@@ -179,7 +191,7 @@ __global__ void __launch_bounds__(NT, S == 4 ? 3 : 1) k_pf_adjoint(const AdjArgs
             q[s].n[k] = inside ? -a.nrm[k][g] : 0.0f;
             q[s].h[k] = 0.0f;
         }
-        if (!qv[s]) continue;
+        if (FIRST || !qv[s]) continue;
         const float f[3] = {a.f[j], a.f[N + j], a.f[2 * N + j]};
         const float *gp = a.dimg + 3 * ((size_t)y * a.W + x);
         const float gr[3] = {gp[0] / S, gp[1] / S, gp[2] / S};
@@ -209,7 +221,7 @@ __global__ void __launch_bounds__(NT, S == 4 ? 3 : 1) k_pf_adjoint(const AdjArgs
         for (int ch = 0; ch < 3; ch++) q[s].h[ch] = f[ch] > 0.0f && f[ch] < 1e5f ? dlum * Y[ch] : 0.0f;
         q[s].nhf = -(q[s].h[0] * f[0] + q[s].h[1] * f[1] + q[s].h[2] * f[2]);
     }
-    reduce(gsum, 0, NG - 3);
+    if (!FIRST) reduce(gsum, 0, NG - 3);
     }
 
     KahanF acc[S][4];
@@ -249,8 +261,8 @@ __global__ void __launch_bounds__(NT, S == 4 ? 3 : 1) k_pf_adjoint(const AdjArgs
             if (dy < -R || dy > R) continue;
             Sums part[S];
             const float *rowp = sm + r * CW * S;
-            if constexpr (S == 4) row4(rowp, plane, lx, R, dy, isx2, isp2, isn, q, part);
-            else row_any<S>(rowp, plane, lx, R, dy, isx2, isp2, isn, q, part);
+            if constexpr (S == 4) row4<FIRST>(rowp, plane, lx, R, dy, isx2, isp2, isn, q, part);
+            else row_any<S, FIRST>(rowp, plane, lx, R, dy, isx2, isp2, isn, q, part);
 #pragma unroll
             for (int s = 0; s < S; s++) {
                 acc[s][0].add(part[s].d);
@@ -258,6 +270,16 @@ __global__ void __launch_bounds__(NT, S == 4 ? 3 : 1) k_pf_adjoint(const AdjArgs
                 for (int k = 0; k < 3; k++) acc[s][k + 1].add(part[s].e[k]);
             }
         }
+    }
+    if constexpr (FIRST) {
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            if (!inside) break;
+            const size_t j = ((size_t)y * a.W + x) * S + s;
+#pragma unroll
+            for (int k = 0; k < 3; k++) a.f[k * N + j] = qv[s] ? acc[s][k + 1].s / acc[s][0].s : 0.0f;
+        }
+        return;
     }
     float bw[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
@@ -334,15 +356,91 @@ __global__ void __launch_bounds__(256) k_reduce_partials(const float *partials, 
     if (t == 0) outv[k] = sum[0];
 }
 
-template <int S>
-sty_status launch_adj(const AdjArgs &a, cudaStream_t st) {
+template <int S, bool FIRST>
+sty_status launch_sweep(const AdjArgs &a, cudaStream_t st) {
     const int CW = TW + 2 * a.R;
     const size_t smem = (size_t)NF * CH * CW * S * sizeof(float);
-    STY_TRY(check_cuda(cudaFuncSetAttribute(k_pf_adjoint<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+    STY_TRY(check_cuda(cudaFuncSetAttribute(k_pf_adjoint<S, FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
                        "attr k_pf_adjoint"));
     const unsigned grid = (unsigned)((a.W + TW - 1) / TW) * (unsigned)((a.H + TH - 1) / TH);
-    k_pf_adjoint<S><<<grid, NT, smem, st>>>(a);
+    k_pf_adjoint<S, FIRST><<<grid, NT, smem, st>>>(a);
     return check_launch("k_pf_adjoint");
+}
+template <bool FIRST>
+sty_status sweep(const AdjArgs &a, int S, cudaStream_t st) {
+    switch (S) {
+        case 1: return launch_sweep<1, FIRST>(a, st);
+        case 2: return launch_sweep<2, FIRST>(a, st);
+        case 4: return launch_sweep<4, FIRST>(a, st);
+        default: return launch_sweep<8, FIRST>(a, st);
+    }
+}
+
+// Whether f_i is formed by the sweep's own operations, so that the sums of w (in_j - f_i) cancel with the weights they are
+// made of, or taken from the forward filter, whose weights are rounded otherwise. Error of the gradient's norm against 64
+// bits with the filter's f, over 39 sets of records and bandwidths, as a multiple of that with the sweep's (geometric mean,
+// largest): 1 sample 1.0, 2.8; 2 samples 1.6, 38 (2.8e-6 for 7e-8); 4 samples (whose filter subtracts a tile's
+// centre from the positions before it scales them) 0.9, 2.1; 8 samples 1.4, 12. The 2.1 and the like are surfaces with
+// sigma_nrm <= 0.05: the filter rounds the normal term's factor into the normals. The first sweep takes
+// 0.9 ms at 512 x 512, 4 spp, radius 8, where the whole is 1.65 without it.
+bool sweep_gives_f(int spp, float sigma_nrm) { return spp == 2 || spp == 8 || sigma_nrm < 0.1f; }
+
+// everything both entry points launch, with their scratch: f 3 N floats, dimg 3 per pixel, parts NG per block, lparts one per
+// 256 pixels, lsum 1
+sty_status run_adjoint(const sty_pf_records *rec, uint32_t depth, int32_t radius, const float prm[36], uint32_t n_steps,
+                       const float *in_next, const float *target, float *f, float *dimg, float *parts, float *lparts, float *lsum,
+                       float *grad, cudaStream_t st) {
+    const int Wd = rec->width, Hd = rec->height, S = rec->spp;
+    const size_t N = (size_t)Wd * Hd * S;
+    const int nb = ((Wd + TW - 1) / TW) * ((Hd + TH - 1) / TH), lb = (Wd * Hd + 255) / 256;
+    // the ramp node (at this depth only), applied to the forward filter's result
+    sty_style_program prog;
+    memset(&prog, 0, sizeof(prog));
+    prog.n_nodes = 1;
+    sty_style_node &nd = prog.nodes[0];
+    nd.kind = STY_STYLE_RAMP_SMOOTH;
+    nd.depth_mask = 1u << (depth > 31 ? 31 : depth);
+    nd.n = (int32_t)n_steps;
+    nd.p[0] = prm[0];
+    for (uint32_t k = 0; k < n_steps; k++) {
+        nd.p[1 + k] = prm[1 + k];
+        for (int c = 0; c < 3; c++) nd.p[9 + 3 * k + c] = prm[9 + 3 * k + c];
+    }
+    AdjArgs a;
+    for (int k = 0; k < 3; k++) {
+        a.pos[k] = rec->pos[k];
+        a.nrm[k] = rec->nrm[k];
+        a.rad[k] = rec->rad[k];
+        a.thr[k] = rec->thr[k];
+    }
+    a.valid = rec->valid;
+    a.in_next = in_next;
+    a.dimg = dimg;
+    a.f = f;
+    a.W = Wd;
+    a.H = Hd;
+    a.R = radius;
+    a.depth = depth;
+    a.sx = prm[33];
+    a.sp = prm[34];
+    a.sn = prm[35];
+    a.s = prm[0];
+    for (int k = 0; k < 8; k++) {
+        a.t[k] = prm[1 + k];
+        for (int c = 0; c < 3; c++) a.c[k][c] = prm[9 + 3 * k + c];
+    }
+    a.nsteps = (int)n_steps;
+    a.partials = parts;
+    const sty_pf_screen_params sp = {radius, prm[33], prm[34], prm[35]};
+    STY_TRY(screen_filter_depth(rec, depth, &sp, nullptr, in_next, f, nullptr, false, st));
+    k_img_loss<<<lb, 256, 0, st>>>(f, rec->valid + (size_t)depth * N, prog, depth, Wd, Hd, S, target, dimg, lparts);
+    STY_TRY(check_launch("k_img_loss"));
+    if (sweep_gives_f(S, prm[35])) STY_TRY(sweep<true>(a, S, st));
+    STY_TRY(sweep<false>(a, S, st));
+    k_reduce_partials<<<NG, 256, 0, st>>>(parts, nb, NG, grad);
+    STY_TRY(check_launch("k_reduce_partials"));
+    k_reduce_partials<<<1, 256, 0, st>>>(lparts, lb, 1, lsum);
+    return check_launch("k_reduce_partials(loss)");
 }
 
 }  // namespace
@@ -363,20 +461,6 @@ extern "C" sty_status sty_pf_adjoint(const sty_pf_records *rec, uint32_t depth, 
     cudaStream_t st = as_stream(stream);
     const int Wd = rec->width, Hd = rec->height, S = rec->spp;
     const size_t N = (size_t)Wd * Hd * S;
-    // forward through the product filter; the ramp node (at this depth only) is applied to its result
-    sty_style_program prog;
-    memset(&prog, 0, sizeof(prog));
-    prog.n_nodes = 1;
-    sty_style_node &nd = prog.nodes[0];
-    nd.kind = STY_STYLE_RAMP_SMOOTH;
-    nd.depth_mask = 1u << (depth > 31 ? 31 : depth);
-    nd.n = (int32_t)n_steps;
-    nd.p[0] = prm[0];
-    for (uint32_t k = 0; k < n_steps; k++) {
-        nd.p[1 + k] = prm[1 + k];
-        for (int c = 0; c < 3; c++) nd.p[9 + 3 * k + c] = prm[9 + 3 * k + c];
-    }
-    sty_pf_screen_params sp = {radius, prm[33], prm[34], prm[35]};
     const int gx = (Wd + TW - 1) / TW, gy = (Hd + TH - 1) / TH, nb = gx * gy;
     const int npix = Wd * Hd, lb = (npix + 255) / 256;
     float *out = nullptr, *dimg = nullptr, *parts = nullptr, *lparts = nullptr, *lsum = nullptr;
@@ -385,52 +469,8 @@ extern "C" sty_status sty_pf_adjoint(const sty_pf_records *rec, uint32_t depth, 
     if (s == STY_OK) s = check_cuda(cudaMallocAsync((void **)&parts, (size_t)nb * NG * 4, st), "alloc partials");
     if (s == STY_OK) s = check_cuda(cudaMallocAsync((void **)&lparts, (size_t)lb * 4, st), "alloc loss partials");
     if (s == STY_OK) s = check_cuda(cudaMallocAsync((void **)&lsum, 4, st), "alloc loss");
-    if (s == STY_OK) s = screen_filter_depth(rec, depth, &sp, nullptr, in_next, out, nullptr, false, stream);
-    if (s == STY_OK) {
-        k_img_loss<<<lb, 256, 0, st>>>(out, rec->valid + (size_t)depth * N, prog, depth, Wd, Hd, S, target, dimg, lparts);
-        s = check_launch("k_img_loss");
-    }
-    if (s == STY_OK) {
-        AdjArgs a;
-        for (int k = 0; k < 3; k++) {
-            a.pos[k] = rec->pos[k];
-            a.nrm[k] = rec->nrm[k];
-            a.rad[k] = rec->rad[k];
-            a.thr[k] = rec->thr[k];
-        }
-        a.valid = rec->valid;
-        a.in_next = in_next;
-        a.dimg = dimg;
-        a.f = out;
-        a.W = Wd;
-        a.H = Hd;
-        a.R = radius;
-        a.depth = depth;
-        a.sx = prm[33];
-        a.sp = prm[34];
-        a.sn = prm[35];
-        a.s = prm[0];
-        for (int k = 0; k < 8; k++) {
-            a.t[k] = prm[1 + k];
-            for (int c = 0; c < 3; c++) a.c[k][c] = prm[9 + 3 * k + c];
-        }
-        a.nsteps = (int)n_steps;
-        a.partials = parts;
-        switch (S) {
-            case 1: s = launch_adj<1>(a, st); break;
-            case 2: s = launch_adj<2>(a, st); break;
-            case 4: s = launch_adj<4>(a, st); break;
-            default: s = launch_adj<8>(a, st); break;
-        }
-    }
-    if (s == STY_OK) {
-        k_reduce_partials<<<NG, 256, 0, st>>>(parts, nb, NG, grad);
-        s = check_launch("k_reduce_partials");
-    }
-    if (s == STY_OK) {
-        k_reduce_partials<<<1, 256, 0, st>>>(lparts, lb, 1, lsum);
-        s = check_launch("k_reduce_partials(loss)");
-    }
+    if (s == STY_OK)
+        s = run_adjoint(rec, depth, radius, prm, n_steps, in_next, target, out, dimg, parts, lparts, lsum, grad, st);
     if (s == STY_OK && loss_out) {
         s = check_cuda(cudaMemcpyAsync(loss_out, lsum, 4, cudaMemcpyDeviceToHost, st), "read loss");
         if (s == STY_OK) s = check_cuda(cudaStreamSynchronize(st), "sync loss");
@@ -507,15 +547,13 @@ extern "C" sty_status sty_pf_adjoint_noalloc(const sty_pf_records *rec, uint32_t
     STY_ARG_CHECK(rec->width > 0 && rec->height > 0, "empty image");
     const int Wd = rec->width, Hd = rec->height, S = rec->spp;
     const size_t N = (size_t)Wd * Hd * S, npix = (size_t)Wd * Hd;
-    const int gx = (Wd + TW - 1) / TW, gy = (Hd + TH - 1) / TH;
-    const size_t nb = (size_t)gx * gy, lb = (npix + 255) / 256;
     STY_ARG_CHECK(N <= kNaMaxRecords,
                   "sty_pf_adjoint_noalloc: %zu records per depth exceed the fixed scratch limit of %zu "
                   "(width * height * spp); use sty_pf_adjoint", N, kNaMaxRecords);
     STY_ARG_CHECK(npix <= kNaMaxPixels,
                   "sty_pf_adjoint_noalloc: %zu pixels exceed the fixed scratch limit of %zu; use sty_pf_adjoint",
                   npix, kNaMaxPixels);
-    const size_t tiles = (size_t)gx * ((Hd + 7) / 8);
+    const size_t tiles = (size_t)((Wd + 31) / 32) * ((Hd + 7) / 8);
     static_assert(TH == 4 && TW == 32, "at most two blocks per tile of 32 x 8 pixels");
     STY_ARG_CHECK(tiles <= kNaMaxBlocks, "sty_pf_adjoint_noalloc: %zu tiles exceed the fixed scratch limit of %zu",
                   tiles, kNaMaxBlocks);
@@ -524,59 +562,9 @@ extern "C" sty_status sty_pf_adjoint_noalloc(const sty_pf_records *rec, uint32_t
     float *out = scratch + kNaOut, *dimg = scratch + kNaDimg, *parts = scratch + kNaParts;
     float *lparts = scratch + kNaLParts, *lsum = scratch + kNaLoss;
     cudaStream_t st = as_stream(stream);
-    sty_style_program prog;
-    memset(&prog, 0, sizeof(prog));
-    prog.n_nodes = 1;
-    sty_style_node &nd = prog.nodes[0];
-    nd.kind = STY_STYLE_RAMP_SMOOTH;
-    nd.depth_mask = 1u << (depth > 31 ? 31 : depth);
-    nd.n = (int32_t)n_steps;
-    nd.p[0] = prm[0];
-    for (uint32_t k = 0; k < n_steps; k++) {
-        nd.p[1 + k] = prm[1 + k];
-        for (int c = 0; c < 3; c++) nd.p[9 + 3 * k + c] = prm[9 + 3 * k + c];
-    }
-    sty_pf_screen_params sp = {radius, prm[33], prm[34], prm[35]};
-    // Every scratch region below is fully overwritten before it is read (no accumulation into
-    // scratch), so nothing has to be cleared between calls.
-    STY_TRY(screen_filter_depth(rec, depth, &sp, nullptr, in_next, out, nullptr, false, stream));
-    k_img_loss<<<(unsigned)lb, 256, 0, st>>>(out, rec->valid + (size_t)depth * N, prog, depth, Wd, Hd, S, target, dimg, lparts);
-    STY_TRY(check_launch("k_img_loss"));
-    AdjArgs a;
-    for (int k = 0; k < 3; k++) {
-        a.pos[k] = rec->pos[k];
-        a.nrm[k] = rec->nrm[k];
-        a.rad[k] = rec->rad[k];
-        a.thr[k] = rec->thr[k];
-    }
-    a.valid = rec->valid;
-    a.in_next = in_next;
-    a.dimg = dimg;
-    a.f = out;
-    a.W = Wd;
-    a.H = Hd;
-    a.R = radius;
-    a.depth = depth;
-    a.sx = prm[33];
-    a.sp = prm[34];
-    a.sn = prm[35];
-    a.s = prm[0];
-    for (int k = 0; k < 8; k++) {
-        a.t[k] = prm[1 + k];
-        for (int c = 0; c < 3; c++) a.c[k][c] = prm[9 + 3 * k + c];
-    }
-    a.nsteps = (int)n_steps;
-    a.partials = parts;
-    switch (S) {
-        case 1: STY_TRY(launch_adj<1>(a, st)); break;
-        case 2: STY_TRY(launch_adj<2>(a, st)); break;
-        case 4: STY_TRY(launch_adj<4>(a, st)); break;
-        default: STY_TRY(launch_adj<8>(a, st)); break;
-    }
-    k_reduce_partials<<<NG, 256, 0, st>>>(parts, (int)nb, NG, grad);
-    STY_TRY(check_launch("k_reduce_partials"));
-    k_reduce_partials<<<1, 256, 0, st>>>(lparts, (int)lb, 1, lsum);
-    STY_TRY(check_launch("k_reduce_partials(loss)"));
+    // Every scratch region is fully overwritten before it is read (no accumulation into scratch), so
+    // nothing has to be cleared between calls.
+    STY_TRY(run_adjoint(rec, depth, radius, prm, n_steps, in_next, target, out, dimg, parts, lparts, lsum, grad, st));
     if (loss_out) {
         STY_TRY(check_cuda(cudaMemcpyAsync(loss_out, lsum, 4, cudaMemcpyDeviceToHost, st), "read loss"));
         STY_TRY(check_cuda(cudaStreamSynchronize(st), "sync loss"));
