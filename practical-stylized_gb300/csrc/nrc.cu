@@ -347,15 +347,18 @@ struct AdamArgs {
     float lr, b1, b2, eps, bc1, bc2, ema_decay, ema_old, ema_new;
     size_t n_hidden;
     uint16_t *img, *img_ema, *img3, *img3_ema;
+    float wide_bound;  // FP32 networks: the counts of weights past it, wide[0] of w and wide[1] of ema
+    uint32_t *wide;
 };
 __device__ __forceinline__ void adam_step(const AdamArgs &o, size_t p, float gr) {
     const float mm = o.b1 * o.m[p] + (1.0f - o.b1) * gr;
     const float vv = o.b2 * o.v[p] + (1.0f - o.b2) * gr * gr;
     o.m[p] = mm;
     o.v[p] = vv;
-    const float wn = o.w[p] - o.lr * (mm / o.bc1) / (sqrtf(vv / o.bc2) + o.eps);
+    const float w0 = o.w[p], e0 = o.ema[p];
+    const float wn = w0 - o.lr * (mm / o.bc1) / (sqrtf(vv / o.bc2) + o.eps);
     o.w[p] = wn;
-    const float en = (o.ema[p] * o.ema_decay * o.ema_old + wn * (1.0f - o.ema_decay)) * o.ema_new;
+    const float en = (e0 * o.ema_decay * o.ema_old + wn * (1.0f - o.ema_decay)) * o.ema_new;
     o.ema[p] = en;
     if (o.img) {
         nrc_store_bf16(o.img, p, wn);
@@ -364,6 +367,12 @@ __device__ __forceinline__ void adam_step(const AdamArgs &o, size_t p, float gr)
     if (o.img3 && p < o.n_hidden) {
         nrc_store_pieces(o.img3, p, wn);
         nrc_store_pieces(o.img3_ema, p, en);
+    }
+    if (o.img3) {
+        const int dw = (int)nrc_is_wide(wn, o.wide_bound) - (int)nrc_is_wide(w0, o.wide_bound);
+        const int de = (int)nrc_is_wide(en, o.wide_bound) - (int)nrc_is_wide(e0, o.wide_bound);
+        if (dw) atomicAdd(o.wide, (uint32_t)dw);
+        if (de) atomicAdd(o.wide + 1, (uint32_t)de);
     }
 }
 
@@ -471,6 +480,7 @@ struct sty_nrc {
     // the same stream, so a call that only reads the network writes nothing.
     uint16_t *img = nullptr, *img_ema = nullptr;
     uint16_t *img3 = nullptr, *img3_ema = nullptr;
+    uint32_t *wide = nullptr;  // how many of w's and of ema's parameters are too wide for the pieces (FP32 networks)
     float *bin = nullptr, *btg = nullptr, *bpred = nullptr, *acts = nullptr, *dpre = nullptr, *loss = nullptr;
     float *gpart = nullptr;  // per-chunk weight-gradient partials
     GridModel *grid = nullptr;  // the composite-encoding network (sty_nrc_create_grid), else null
@@ -574,8 +584,8 @@ sty_status pack_images(sty_nrc *nr, cudaStream_t st) {
         STY_TRY(nrc_tc_pack(nr->net, nr->ema, nr->img_ema, st));
     }
     if (nr->img3) {
-        STY_TRY(nrc_f32tc_pack(nr->net, nr->w, nr->img3, st));
-        STY_TRY(nrc_f32tc_pack(nr->net, nr->ema, nr->img3_ema, st));
+        STY_TRY(nrc_f32tc_pack(nr->net, nr->w, nr->img3, nr->wide, st));
+        STY_TRY(nrc_f32tc_pack(nr->net, nr->ema, nr->img3_ema, nr->wide + 1, st));
     }
     return STY_OK;
 }
@@ -589,13 +599,14 @@ sty_status infer(sty_nrc *nr, bool ema, uint64_t count, const float *in, float *
     }
     if (nr->cfg.precision == STY_NRC_BF16)
         return nrc_tc_forward(nr->net, ema ? nr->img_ema : nr->img, count, in, out, st);
-    return nrc_f32tc_forward(nr->net, ema ? nr->ema : nr->w, ema ? nr->img3_ema : nr->img3, count, in, out, st);
+    return nrc_f32tc_forward(nr->net, ema ? nr->ema : nr->w, ema ? nr->img3_ema : nr->img3, nr->wide + (ema ? 1 : 0), count, in, out,
+                             st);
 }
 
 void free_nrc(sty_nrc *nr) {
     grid_destroy(nr->grid);
     void *ptrs[] = {nr->w, nr->m, nr->v, nr->g, nr->ema, nr->img, nr->img_ema, nr->bin,
-                    nr->btg, nr->bpred, nr->acts, nr->dpre, nr->loss, nr->gpart, nr->img3, nr->img3_ema};
+                    nr->btg, nr->bpred, nr->acts, nr->dpre, nr->loss, nr->gpart, nr->img3, nr->img3_ema, nr->wide};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     delete nr;
@@ -642,6 +653,7 @@ sty_status sty_nrc_create(const sty_nrc_config *cfg, sty_nrc **out) {
     if (cfg->precision == STY_NRC_FP32) {
         alloc((void **)&nr->img3, nrc_f32tc_image_elems(nr->net) * 2, "alloc piece images");
         alloc((void **)&nr->img3_ema, nrc_f32tc_image_elems(nr->net) * 2, "alloc ema piece images");
+        alloc((void **)&nr->wide, 8, "alloc wide weights");
     }
     if (s == STY_OK) s = ensure_batch(nr, cfg->batch_size);
     if (s == STY_OK) {
@@ -845,7 +857,8 @@ sty_status sty_nrc_train(sty_nrc *nr, uint64_t count, uint64_t n_iters, const fl
             nr->img_dirty = true;
         } else {
             const AdamArgs o = {nr->w, nr->m, nr->v, nr->ema, lr_t, c.beta1, c.beta2, c.epsilon, bc1, bc2, c.ema_decay,
-                                ema_old, ema_new, nrc_w_offset(nr->net.layers), nr->img, nr->img_ema, nr->img3, nr->img3_ema};
+                                ema_old, ema_new, nrc_w_offset(nr->net.layers), nr->img, nr->img_ema, nr->img3, nr->img3_ema,
+                                nrc_wide_bound(nr->net), nr->wide};
             STY_TRY(sum_chunks<true>(nr->np, chunks, nr->gpart, nullptr, o, st));
         }
     }

@@ -151,9 +151,15 @@ __device__ __forceinline__ void nrc_store_pieces(uint16_t *img, size_t i, float 
         if (p == 1) r = fmaf(v, kNrcUnbias, r);
     }
 }
-sty_status nrc_f32tc_pack(const NrcNet &n, const float *w, uint16_t *img, cudaStream_t st);
-sty_status nrc_f32tc_forward(const NrcNet &n, const float *w, const uint16_t *img, uint64_t count, const float *input,
-                             float *output, cudaStream_t st);
+// Where a piece or a sum could leave FP32's range the pieces do not add up (the first one of an infinity leaves a NaN behind
+// it), so a network that holds a weight past this bound, or a NaN, is run row by row on the CUDA cores: with every weight
+// of L + 1 matrices within it, each matrix multiplies the range of |activations| <= 1 by at most 64 times it, 2^120 in all.
+// `wide` counts such weights; whoever writes a parameter keeps the count.
+inline float nrc_wide_bound(const NrcNet &n) { return exp2f(120.0f / (float)(n.layers + 1) - 6.0f); }
+__device__ __forceinline__ bool nrc_is_wide(float v, float bound) { return !(fabsf(v) <= bound); }
+sty_status nrc_f32tc_pack(const NrcNet &n, const float *w, uint16_t *img, uint32_t *wide, cudaStream_t st);
+sty_status nrc_f32tc_forward(const NrcNet &n, const float *w, const uint16_t *img, const uint32_t *wide, uint64_t count,
+                             const float *input, float *output, cudaStream_t st);
 // The reference's composite-encoding network (nrc_grid.cu)
 struct GridModel;
 sty_status grid_create(const sty_nrc_grid_config *c, GridModel **out, size_t *n_params, size_t *n_mlp);

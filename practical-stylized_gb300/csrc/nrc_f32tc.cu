@@ -47,16 +47,21 @@ constexpr uint32_t kImg = W * W * 2;          // bytes of one piece of a layer
 constexpr uint32_t kLayer = 3 * kImg;         // w1, w2, w3
 
 
-__global__ void k_pack3(int layers, const float *__restrict__ w, uint16_t *__restrict__ img) {
+__global__ void k_pack3(int layers, uint32_t np, float bound, const float *__restrict__ w, uint16_t *__restrict__ img,
+                        uint32_t *__restrict__ wide) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < (uint32_t)layers * W * W) nrc_store_pieces(img, i, w[i]);
+    if (i >= np) return;
+    const float v = w[i];
+    if (i < (uint32_t)layers * W * W) nrc_store_pieces(img, i, v);
+    if (nrc_is_wide(v, bound)) atomicAdd(wide, 1u);
 }
 
 struct Args {
     NrcNet n;
     int c4;
     const uint16_t *img;
-    const float *wout;  // FP32 output layer
+    const float *w;        // FP32 parameters
+    const uint32_t *wide;  // nrc_is_wide weights among them
     uint64_t count;
     const float *input;
     float *output;
@@ -123,6 +128,27 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
                  : "r"(taddr));
 }
 
+// A network with wide weights: every row by one thread, each sum over k = 0 .. 63 in order with fmaf, so that what overflows
+// does as it does in FP32 (the bits of the CUDA-core kernel that this one replaced).
+__device__ __noinline__ void rows_f32(const Args &a) {
+    float buf[2][W];
+    for (uint64_t row = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; row < a.count; row += (uint64_t)gridDim.x * blockDim.x) {
+        nrc_encode(a.n, a.input + row * a.n.in_dims, buf[0]);
+        for (int l = 0; l <= a.n.layers; l++) {
+            const bool out = l == a.n.layers;
+            const float *h = buf[l & 1], *w = a.w + nrc_w_offset(l);
+            for (int j = 0; j < (out ? a.n.out_dims : W); j++, w += W) {
+                float s = 0.0f;
+                for (int k = 0; k < W; k++) s = fmaf(w[k], h[k], s);
+                if (out)
+                    a.output[row * a.n.out_dims + j] = s;
+                else
+                    buf[(l + 1) & 1][j] = fmaxf(s, 0.0f);
+            }
+        }
+    }
+}
+
 // OM: output columns kept in registers (4, or 16 for wider outputs)
 template <int OM>
 __global__ void __launch_bounds__(kGT * kTiles, 1) k_nrc_f32tc(const Args a) {
@@ -134,7 +160,8 @@ __global__ void __launch_bounds__(kGT * kTiles, 1) k_nrc_f32tc(const Args a) {
     const bool issuer = warp % (kGT / 32) == 0;  // the tile's issuing warp
     const uint32_t bar_id = 1u + (uint32_t)grp;
     const int L = a.n.layers, O = a.n.out_dims;
-    for (int e = tid; e < O * W; e += kGT * kTiles) wo[e] = a.wout[e];
+    const uint32_t wide = *reinterpret_cast<const volatile uint32_t *>(a.wide);
+    for (int e = tid; e < O * W; e += kGT * kTiles) wo[e] = a.w[nrc_w_offset(L) + e];
     if (tid == 0) {
         for (int g = 0; g < kTiles; g++)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar[g])) : "memory");
@@ -198,7 +225,8 @@ __global__ void __launch_bounds__(kGT * kTiles, 1) k_nrc_f32tc(const Args a) {
     };
 
     bool loaded = false;  // the weight images have arrived
-    const uint64_t ntiles = (a.count + TM - 1) / TM;
+    const uint64_t ntiles = wide ? 0 : (a.count + TM - 1) / TM;
+    if (wide) rows_f32(a);
     // the workload encoder's inputs of this thread's half, loaded a tile ahead (asm volatile: not sunk to
     // their use)
     float xr[kNrcC4Half];
@@ -326,17 +354,19 @@ sty_status launch(Args a, cudaStream_t st) {
 }  // namespace
 
 size_t nrc_f32tc_image_elems(const NrcNet &n) { return (size_t)n.layers * 3 * W * W; }
-sty_status nrc_f32tc_pack(const NrcNet &n, const float *w, uint16_t *img, cudaStream_t st) {
-    const uint32_t total = (uint32_t)n.layers * W * W;
-    k_pack3<<<(total + 255) / 256, 256, 0, st>>>(n.layers, w, img);
+sty_status nrc_f32tc_pack(const NrcNet &n, const float *w, uint16_t *img, uint32_t *wide, cudaStream_t st) {
+    const uint32_t np = (uint32_t)nrc_param_count(n);
+    STY_TRY(check_cuda(cudaMemsetAsync(wide, 0, 4, st), "zero wide weights"));
+    k_pack3<<<(np + 255) / 256, 256, 0, st>>>(n.layers, np, nrc_wide_bound(n), w, img, wide);
     return check_launch("k_pack3");
 }
-sty_status nrc_f32tc_forward(const NrcNet &n, const float *w, const uint16_t *img, uint64_t count, const float *input,
-                             float *output, cudaStream_t st) {
+sty_status nrc_f32tc_forward(const NrcNet &n, const float *w, const uint16_t *img, const uint32_t *wide, uint64_t count,
+                             const float *input, float *output, cudaStream_t st) {
     Args a{};
     a.n = n;
     a.img = img;
-    a.wout = w + nrc_w_offset(n.layers);
+    a.w = w;
+    a.wide = wide;
     a.count = count;
     a.input = input;
     a.output = output;
