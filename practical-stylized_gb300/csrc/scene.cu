@@ -11,6 +11,7 @@
 #include "scene.cuh"
 
 using namespace sty;
+using namespace sty::bvh;
 
 struct sty_scene {
     uint32_t n_tris = 0, n_materials = 0, n_lights = 0;
@@ -54,220 +55,6 @@ SceneView scene_view(const sty_scene *s) {
 }  // namespace sty
 
 namespace {
-
-struct Box {
-    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-    void grow(const float *p) {
-        for (int a = 0; a < 3; a++) {
-            mn[a] = std::min(mn[a], p[a]);
-            mx[a] = std::max(mx[a], p[a]);
-        }
-    }
-    void grow(const Box &b) {
-        for (int a = 0; a < 3; a++) {
-            mn[a] = std::min(mn[a], b.mn[a]);
-            mx[a] = std::max(mx[a], b.mx[a]);
-        }
-    }
-    float area() const {
-        float d[3];
-        for (int a = 0; a < 3; a++) d[a] = std::max(0.0f, mx[a] - mn[a]);
-        return 2.0f * (d[0] * d[1] + d[1] * d[2] + d[2] * d[0]);
-    }
-};
-
-struct Node2 {
-    float bmin[3], bmax[3];
-    uint32_t a;      // internal: left child (right = a + 1); leaf: first triangle slot
-    uint32_t count;  // 0 = internal, else number of triangles in the leaf
-    float area() const {
-        float d[3];
-        for (int k = 0; k < 3; k++) d[k] = std::max(0.0f, bmax[k] - bmin[k]);
-        return d[0] * d[1] + d[1] * d[2] + d[2] * d[0];
-    }
-};
-
-// Binned SAH (16 bins per axis), leaves of at most 4 triangles.
-struct Builder {
-    const float *pos;
-    std::vector<Box> tbox;
-    std::vector<float> cent;  // 3 per triangle
-    std::vector<uint32_t> idx;
-    std::vector<Node2> nodes;
-
-    void build(uint32_t n) {
-        tbox.resize(n);
-        cent.resize(3 * (size_t)n);
-        idx.resize(n);
-        for (uint32_t i = 0; i < n; i++) {
-            for (int v = 0; v < 3; v++) tbox[i].grow(pos + 9 * (size_t)i + 3 * v);
-            for (int a = 0; a < 3; a++) cent[3 * (size_t)i + a] = 0.5f * (tbox[i].mn[a] + tbox[i].mx[a]);
-            idx[i] = i;
-        }
-        nodes.reserve(2 * (size_t)n);
-        nodes.push_back(Node2());
-        subdivide(0, 0, n);
-    }
-    void set_bounds(Node2 &nd, uint32_t b, uint32_t e) {
-        Box bx;
-        for (uint32_t i = b; i < e; i++) bx.grow(tbox[idx[i]]);
-        for (int a = 0; a < 3; a++) {
-            nd.bmin[a] = bx.mn[a];
-            nd.bmax[a] = bx.mx[a];
-        }
-    }
-    void subdivide(uint32_t ni, uint32_t b, uint32_t e) {
-        set_bounds(nodes[ni], b, e);
-        const uint32_t cnt = e - b;
-        if (cnt <= 4) {
-            nodes[ni].a = b;
-            nodes[ni].count = cnt;
-            return;
-        }
-        Box cb;
-        for (uint32_t i = b; i < e; i++) cb.grow(&cent[3 * (size_t)idx[i]]);
-        constexpr int NB = 16;
-        float best = INFINITY;
-        int best_axis = -1, best_bin = 0;
-        for (int a = 0; a < 3; a++) {
-            const float ext = cb.mx[a] - cb.mn[a];
-            if (!(ext > 0.0f)) continue;
-            Box bins[NB];
-            uint32_t counts[NB] = {0};
-            for (uint32_t i = b; i < e; i++) {
-                int k = (int)((cent[3 * (size_t)idx[i] + a] - cb.mn[a]) / ext * NB);
-                k = std::min(std::max(k, 0), NB - 1);
-                bins[k].grow(tbox[idx[i]]);
-                counts[k]++;
-            }
-            float la[NB], ra[NB];
-            uint32_t lc[NB], rc[NB];
-            Box acc;
-            uint32_t c = 0;
-            for (int k = 0; k < NB; k++) {
-                acc.grow(bins[k]);
-                c += counts[k];
-                la[k] = acc.area();
-                lc[k] = c;
-            }
-            acc = Box();
-            c = 0;
-            for (int k = NB - 1; k >= 0; k--) {
-                acc.grow(bins[k]);
-                c += counts[k];
-                ra[k] = acc.area();
-                rc[k] = c;
-            }
-            for (int k = 0; k < NB - 1; k++) {
-                if (lc[k] == 0 || rc[k + 1] == 0) continue;
-                const float cost = la[k] * lc[k] + ra[k + 1] * rc[k + 1];
-                if (cost < best) {
-                    best = cost;
-                    best_axis = a;
-                    best_bin = k;
-                }
-            }
-        }
-        uint32_t mid;
-        if (best_axis < 0) {
-            mid = b + cnt / 2;  // degenerate centroids: split by index
-        } else {
-            const float ext = cb.mx[best_axis] - cb.mn[best_axis];
-            auto it = std::partition(idx.begin() + b, idx.begin() + e, [&](uint32_t t) {
-                int k = (int)((cent[3 * (size_t)t + best_axis] - cb.mn[best_axis]) / ext * NB);
-                k = std::min(std::max(k, 0), NB - 1);
-                return k <= best_bin;
-            });
-            mid = (uint32_t)(it - idx.begin());
-            if (mid == b || mid == e) mid = b + cnt / 2;
-        }
-        const uint32_t l = (uint32_t)nodes.size();
-        nodes.push_back(Node2());
-        nodes.push_back(Node2());
-        nodes[ni].a = l;
-        nodes[ni].count = 0;
-        subdivide(l, b, mid);
-        subdivide(l + 1, mid, e);
-    }
-};
-
-// The binary tree as 4-wide nodes (each takes its two children and opens the larger of them, by
-// surface, until it has `width`), the children's boxes quantised to the node's grid. Breadth first, so the
-// top of the tree is contiguous.
-std::vector<BvhNode> widen(const std::vector<Node2> &n2, int width, int *stack) {
-    std::vector<BvhNode> out(1);
-    std::vector<int> held(1, 0);  // entries on a walk's stack at most when it comes to the node
-    *stack = 0;
-    std::vector<uint32_t> src(1, 0);  // the binary node each wide node was made from
-    out.reserve(n2.size() / 2 + 1);
-    for (size_t i = 0; i < src.size(); i++) {
-        uint32_t kid[4];
-        int nk = 0;
-        const Node2 &root = n2[src[i]];
-        if (root.count) {  // a one-leaf tree
-            kid[nk++] = src[i];
-        } else {
-            kid[nk++] = root.a;
-            kid[nk++] = root.a + 1;
-            while (nk < width) {
-                int best = -1;
-                for (int k = 0; k < nk; k++)
-                    if (!n2[kid[k]].count && (best < 0 || n2[kid[k]].area() > n2[kid[best]].area())) best = k;
-                if (best < 0) break;
-                const uint32_t a = n2[kid[best]].a;
-                kid[best] = a;
-                kid[nk++] = a + 1;
-            }
-        }
-        const int holds = held[i] + nk - 1;
-        *stack = std::max(*stack, holds);
-        BvhNode w;
-        memset(&w, 0, sizeof(w));
-        w.exp = (uint32_t)nk << 24;
-        for (int a = 0; a < 3; a++) {
-            float lo = n2[kid[0]].bmin[a], hi = n2[kid[0]].bmax[a];
-            for (int k = 1; k < nk; k++) {
-                lo = std::min(lo, n2[kid[k]].bmin[a]);
-                hi = std::max(hi, n2[kid[k]].bmax[a]);
-            }
-            if (!std::isfinite(lo) || !std::isfinite(hi)) {  // no grid holds the box: an axis that excludes nothing
-                w.o[a] = -0x1p127f;
-                w.exp |= 254u << (8 * a);
-                w.hi[a] = 0xffffffffu;
-                continue;
-            }
-            // spacing: 250 steps cover the box; not below 2^-20 of the coordinates, whose own rounding the
-            // corner has
-            const double mag = std::max(std::fabs((double)lo), std::fabs((double)hi));
-            const double need = std::max(std::max(((double)hi - lo) / 250.0, mag * 0x1p-20), 0x1p-100);
-            int e;
-            std::frexp(need, &e);  // need <= 2^e
-            const double step = std::ldexp(1.0, e);
-            w.o[a] = (float)((double)lo - 2.0 * step);
-            w.exp |= (uint32_t)(e + 127) << (8 * a);
-            for (int k = 0; k < nk; k++) {
-                const double ql = std::floor(((double)n2[kid[k]].bmin[a] - w.o[a]) / step) - 1.0;
-                const double qh = std::ceil(((double)n2[kid[k]].bmax[a] - w.o[a]) / step) + 1.0;
-                w.lo[a] |= (uint32_t)std::min(std::max(0.0, ql), 255.0) << (8 * k);
-                w.hi[a] |= (uint32_t)std::min(std::max(0.0, qh), 255.0) << (8 * k);
-            }
-        }
-        for (int k = 0; k < nk; k++) {
-            const Node2 &c = n2[kid[k]];
-            if (c.count) {
-                w.child[k] = c.a;
-                w.count |= c.count << (8 * k);
-            } else {
-                w.child[k] = (uint32_t)src.size();
-                src.push_back(kid[k]);
-                held.push_back(holds);
-                out.emplace_back();
-            }
-        }
-        out[i] = w;
-    }
-    return out;
-}
 
 void free_scene(sty_scene *s) {
     render_cache_free(s->render_cache);
@@ -375,9 +162,8 @@ sty_status sty_scene_create(const float *pos, const uint32_t *tmat, uint32_t n, 
         st = check_cuda(cudaMalloc(dst, bytes), what);
         if (st == STY_OK) st = check_cuda(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice), what);
     };
-    // A wide node leaves up to three entries on the stack per level: a tree too deep for that gets narrower nodes.
-    std::vector<BvhNode> wide;
-    for (int width = 4, stack = kStack + 1; width >= 2 && stack > kStack; width--) wide = widen(b.nodes, width, &stack);
+    int stack = 0, width = 0;
+    const std::vector<BvhNode> wide = build_wide(b.nodes, &stack, &width);
     up((void **)&s->nodes, wide.data(), wide.size() * sizeof(BvhNode), "upload bvh");
     up((void **)&s->tris, tg.data(), tg.size() * sizeof(TriGeom), "upload triangles");
     up((void **)&s->tri_material, tmat, n * 4, "upload materials ids");

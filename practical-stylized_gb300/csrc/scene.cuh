@@ -1,25 +1,10 @@
 // scene.cuh -- device view of a scene: 4-wide BVH nodes, triangles, materials; watertight intersection.
 #pragma once
 
+#include "bvh.cuh"
 #include "common.cuh"
 
 namespace sty {
-
-// 4-wide BVH node, 64 bytes. The children's boxes are 8-bit coordinates on the node's own grid, corner
-// `o` and spacing 2^(exp - 127) per axis, rounded outwards and widened by one more grid step, so a box
-// computed from them contains the exact one with a margin above the rounding of the slab test.
-// A step of the walk reads one 64-byte node where the binary tree's read three of 32 bytes, and tests four
-// boxes: 2 M random rays in a room of 49.6 k triangles 22.1 ms with the binary tree, now 2.1.
-struct BvhNode {
-    float o[3];
-    uint32_t exp;       // biased exponent of the spacing, byte a for axis a; byte 3: number of children
-    uint32_t lo[3];     // byte c: child c's lower coordinate
-    uint32_t hi[3];
-    uint32_t child[4];  // internal: node index; leaf: first triangle slot
-    uint32_t count;     // byte c: child c's triangles, 0 = internal
-    uint32_t pad;
-};
-static_assert(sizeof(BvhNode) == 64, "node size");
 
 struct TriGeom {        // 48 bytes, triangle slot order (BVH leaf order)
     float4 v0;          // w = original triangle id (as bits)
@@ -207,7 +192,6 @@ __device__ __forceinline__ uint32_t node_child(const NodeData &n, int c) {
 // One ray's walk through the tree. Stack entries: node index or first triangle slot, and the entry distance
 // with the triangle count (0: a node) in its last 3 bits (rounded down, so nothing is culled that would
 // not have been). `ex0`, `ex1`: original ids skipped.
-constexpr int kStack = 96;
 struct Walk {
     RayPre rp;
     RayBox rb;
