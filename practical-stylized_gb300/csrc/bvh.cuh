@@ -225,7 +225,7 @@ inline std::vector<BvhNode> widen(const std::vector<Node2> &n2, int width, int *
                 lo = std::min(lo, n2[kid[k]].bmin[a]);
                 hi = std::max(hi, n2[kid[k]].bmax[a]);
             }
-            if (!std::isfinite(lo) || !std::isfinite(hi)) {  // no grid holds the box: an axis that excludes nothing
+            if (!(lo >= -0x1p126f && hi <= 0x1p126f)) {  // no grid holds the box: an axis that excludes nothing
                 w.o[a] = -0x1p127f;
                 w.exp |= 254u << (8 * a);
                 w.hi[a] = 0xffffffffu;

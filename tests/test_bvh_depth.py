@@ -84,6 +84,12 @@ def _soup():
     return (rng.uniform(-1, 1, (3000, 1, 3)) + rng.normal(scale=0.05, size=(3000, 3, 3))).astype(np.float32).reshape(-1, 9)
 
 
+def _far(value):
+    pos = _soup()[:200].copy()
+    pos[7, 3] = value  # one vertex at the end of FP32's range
+    return pos
+
+
 # geometry -> the width its tree is given (0: any)
 CASES = {
     "soup": (_soup, 4),
@@ -91,6 +97,8 @@ CASES = {
     "five the same": (lambda: np.repeat(_soup()[:1], 5, 0), 4),
     "halves": (lambda: _nested(0.5, 2.0 ** 100, 2.0 ** -119), 2),
     "halves, fewer": (lambda: _nested(0.5, 2.0 ** 50, 2.0 ** -30), 3),
+    "far": (lambda: _far(3.4e38), 0),
+    "far below": (lambda: _far(-3.4e38), 0),
     "tenths off": (lambda: _nested(0.9, 1e30, 1e-36), 0),
     "a twentieth off": (lambda: _nested(0.95, 1e37, 1e-37), 0),
 }
@@ -141,4 +149,24 @@ def test_hits(sty, cuda, name):
     assert hit.mean() > 0.8
     assert (prim.cpu().numpy().view(np.uint32) == rp).all()
     assert (t.cpu().numpy()[hit] == rt[hit]).all() and (bary.cpu().numpy()[hit] == rb[hit]).all()
+    sc.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [3.4e38, -3.4e38, 1e30])
+def test_hits_beside_a_far_vertex(sty, cuda, value):
+    """A triangle that reaches to the end of the range hides none of the others."""
+    import torch
+    pos = _far(value)
+    rng = np.random.default_rng(3)
+    aim = pos[rng.integers(8, len(pos), 3000)].reshape(-1, 3, 3).mean(1)
+    o = aim + rng.normal(size=(3000, 3))
+    d = (aim - o) / np.linalg.norm(aim - o, axis=1, keepdims=True)
+    rays = np.concatenate([o, d, np.zeros((3000, 1)), np.full((3000, 1), 1e20)], 1).astype(np.float32)
+    _, _, mats, cam = sty.scene.cornell_box(8, 8)
+    sc = sty.scene.Scene(pos, np.zeros(len(pos), np.uint32), mats, cam)
+    prim, t, bary = sc.closest_hit(torch.from_numpy(rays).cuda())
+    rp, rt, rb = oracle.closest_hit(pos, rays)
+    assert (rp != 0xFFFFFFFF).mean() > 0.9
+    assert (prim.cpu().numpy().view(np.uint32) == rp).all()
     sc.close()
