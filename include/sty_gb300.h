@@ -530,6 +530,11 @@ STY_API sty_status sty_scene_create(const float *tri_positions, const uint32_t *
                                     const sty_scene_material *materials, uint32_t n_materials,
                                     const sty_camera *camera, sty_scene **out);
 STY_API sty_status sty_scene_destroy(sty_scene *scene);
+/* Gives back the device memory a scene keeps between calls for the next one of the same kind: the buffers of its last render
+ * and one vertex-tree workspace of sty_brpt_render of at most 8 GB. The next render allocates again. The library does it by
+ * itself for the workspaces of all scenes when one of its own allocations finds memory short, and with the scene; not for
+ * allocations made outside it. Call it with no work of the scene in flight. */
+STY_API sty_status sty_scene_trim(sty_scene *scene);
 /* Closest hit of n rays (device, 8 floats per ray: origin, direction, tmin, tmax). Outputs
  * (device): prim (UINT32_MAX on a miss), t, bary (2 per ray: weights of v1 and v2). The ray query
  * the reference's integrators issue through LuisaCompute (`accel.intersect`), exposed for
@@ -709,7 +714,9 @@ STY_API sty_status sty_pf_nrc_render(sty_scene *scene, sty_nrc *nrc, const sty_p
  * style(Le + mean over branches of (direct + throughput * child radiance * child emission MIS)),
  * the depth-0 radiance is the pixel sample (the non-debiased estimator; the jackknife / Russian-
  * roulette debiasing option is not built). Pixel samples (pixel x repeat) go through in passes
- * whose worst-case vertex trees fit vram_mb (100 bytes per vertex slot). Adds (1/repeats) of each pixel's sample into
+ * whose worst-case vertex trees fit vram_mb (100 bytes per vertex slot); the scene keeps that
+ * workspace, if it is at most 8 GB, for its next call (sty_scene_trim gives it back; a call with a
+ * smaller vram_mb replaces it). Adds (1/repeats) of each pixel's sample into
  * `film` (device, width*height*3 doubles; the caller zeroes it). `programs` is a HOST array.
  * Sampling keys on (seed, repeat, pixel) and, per child, on (parent, branch index): the image does
  * not depend on vram_mb. Deterministic. */

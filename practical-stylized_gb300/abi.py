@@ -113,6 +113,7 @@ SIGNATURES = {
                                            C.POINTER(C.c_float), _VP]),
     "sty_scene_create": (C.c_int32, [_VP, _VP, C.c_uint32, _VP, C.c_uint32, _VP, C.POINTER(C.c_void_p)]),
     "sty_scene_destroy": (C.c_int32, [C.c_void_p]),
+    "sty_scene_trim": (C.c_int32, [C.c_void_p]),
     "sty_scene_closest_hit": (C.c_int32, [C.c_void_p, _VP, C.c_uint64, _VP, _VP, _VP, _VP]),
     "sty_pf_render": (C.c_int32, [C.c_void_p, _VP, _VP, C.c_uint32, _VP, C.POINTER(C.c_uint64), _VP]),
     "sty_nrc_samples": (C.c_int32, [C.c_void_p, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint64, _VP, _VP,

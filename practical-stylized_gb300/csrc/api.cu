@@ -23,6 +23,23 @@ void set_error(const char *fmt, ...) {
 void clear_error() { g_last_error[0] = 0; }
 void count_launch(uint64_t n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
+namespace {
+template <class Alloc>
+cudaError_t alloc_or_release(Alloc alloc) {
+    cudaError_t e = alloc();
+    if (e == cudaErrorMemoryAllocation && release_workspaces()) {
+        cudaGetLastError();
+        e = alloc();
+    }
+    return e;
+}
+}  // namespace
+cudaError_t device_malloc_bytes(void **p, size_t bytes) {
+    return alloc_or_release([&] { return cudaMalloc(p, bytes); });
+}
+cudaError_t device_malloc_async_bytes(void **p, size_t bytes, cudaStream_t st) {
+    return alloc_or_release([&] { return cudaMallocAsync(p, bytes, st); });
+}
 sty_status check_cuda(cudaError_t e, const char *what) {
     if (e == cudaSuccess) return STY_OK;
     set_error("%s: %s (%s)", what, cudaGetErrorString(e), cudaGetErrorName(e));

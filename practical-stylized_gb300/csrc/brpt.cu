@@ -429,7 +429,7 @@ sty_status sty_brpt_render(sty_scene *scene, const sty_brpt_config *cfg, const s
                  o_scan = place(scan_bytes);
     void *ws = nullptr;
     size_t ws_bytes = 0;
-    STY_TRY(scene_take_workspace(scene, at, &ws, &ws_bytes));
+    STY_TRY(scene_take_workspace(scene, at, (size_t)cfg->vram_mb << 20, &ws, &ws_bytes));
     auto cleanup = [&]() { scene_give_workspace(scene, ws, ws_bytes); };
     char *const wp = static_cast<char *>(ws);
     BrSlots sl;

@@ -84,7 +84,7 @@ const float *principled_table() {
     if (it != tables.end()) return it->second;
     float *t = nullptr;
     const int cells = bsdf::kTabN * bsdf::kTabN * bsdf::kTabN;
-    if (cudaMalloc(&t, cells * sizeof(float)) != cudaSuccess) return nullptr;
+    if (device_malloc(&t, cells * sizeof(float)) != cudaSuccess) return nullptr;
     k_ggx_table<<<cells, 256>>>(t);
     count_launch();
     if (cudaDeviceSynchronize() != cudaSuccess) {

@@ -30,6 +30,19 @@ inline cudaStream_t as_stream(void *s) { return reinterpret_cast<cudaStream_t>(s
 // Checks the launch that was just issued; returns STY_ERR_CUDA with the CUDA message on failure.
 sty_status check_launch(const char *what);
 sty_status check_cuda(cudaError_t e, const char *what);
+// cudaMalloc and cudaMallocAsync that, where memory is short, try again once the workspaces that scenes keep between calls
+// have been given back
+cudaError_t device_malloc_bytes(void **p, size_t bytes);
+cudaError_t device_malloc_async_bytes(void **p, size_t bytes, cudaStream_t st);
+template <typename T>
+cudaError_t device_malloc(T **p, size_t bytes) {
+    return device_malloc_bytes(reinterpret_cast<void **>(p), bytes);
+}
+template <typename T>
+cudaError_t device_malloc_async(T **p, size_t bytes, cudaStream_t st) {
+    return device_malloc_async_bytes(reinterpret_cast<void **>(p), bytes, st);
+}
+bool release_workspaces();  // (scene.cu) frees them; false if there were none
 
 #define STY_ARG_CHECK(cond, ...)              \
     do {                                      \

@@ -510,17 +510,17 @@ sty_status ensure_batch(sty_nrc *nr, uint32_t B) {
     nr->bin = nr->btg = nr->bpred = nr->acts = nr->dpre = nr->gpart = nullptr;
     const NrcNet &n = nr->net;
     if (nr->grid) {  // the composite-encoding network: a gathered batch, no partials
-        STY_TRY(check_cuda(cudaMalloc(&nr->bin, (size_t)B * n.in_dims * 4), "alloc batch input"));
-        STY_TRY(check_cuda(cudaMalloc(&nr->btg, (size_t)B * n.out_dims * 4), "alloc batch target"));
+        STY_TRY(check_cuda(device_malloc(&nr->bin, (size_t)B * n.in_dims * 4), "alloc batch input"));
+        STY_TRY(check_cuda(device_malloc(&nr->btg, (size_t)B * n.out_dims * 4), "alloc batch target"));
     } else {
         if (!tc_training(nr)) {
-            STY_TRY(check_cuda(cudaMalloc(&nr->bpred, (size_t)B * n.out_dims * 4), "alloc batch pred"));
-            STY_TRY(check_cuda(cudaMalloc(&nr->acts, (size_t)(n.layers + 1) * B * kNrcWidth * 4), "alloc activations"));
-            STY_TRY(check_cuda(cudaMalloc(&nr->dpre, (size_t)(n.layers + 1) * B * kNrcWidth * 4), "alloc gradients"));
+            STY_TRY(check_cuda(device_malloc(&nr->bpred, (size_t)B * n.out_dims * 4), "alloc batch pred"));
+            STY_TRY(check_cuda(device_malloc(&nr->acts, (size_t)(n.layers + 1) * B * kNrcWidth * 4), "alloc activations"));
+            STY_TRY(check_cuda(device_malloc(&nr->dpre, (size_t)(n.layers + 1) * B * kNrcWidth * 4), "alloc gradients"));
         }
         size_t chunks = (B + kWgChunk - 1) / kWgChunk;
         if (nr->cfg.precision == STY_NRC_BF16) chunks = std::max<size_t>(chunks, nrc_tc_train_ctas(B));
-        STY_TRY(check_cuda(cudaMalloc(&nr->gpart, chunks * nr->np * 4), "alloc gradient partials"));
+        STY_TRY(check_cuda(device_malloc(&nr->gpart, chunks * nr->np * 4), "alloc gradient partials"));
     }
     nr->bcap = B;
     return STY_OK;
@@ -639,7 +639,7 @@ sty_status sty_nrc_create(const sty_nrc_config *cfg, sty_nrc **out) {
     nr->lr = cfg->learning_rate;
     sty_status s = STY_OK;
     auto alloc = [&](void **p, size_t bytes, const char *what) {
-        if (s == STY_OK) s = check_cuda(cudaMalloc(p, bytes), what);
+        if (s == STY_OK) s = check_cuda(device_malloc(p, bytes), what);
     };
     alloc((void **)&nr->w, nr->np * 4, "alloc weights");
     alloc((void **)&nr->m, nr->np * 4, "alloc adam m");
@@ -709,7 +709,7 @@ sty_status sty_nrc_create_grid(const sty_nrc_grid_config *gc, sty_nrc **out) {
     nr->np = np;
     nr->lr = gc->learning_rate;
     auto alloc = [&](void **p, size_t bytes, const char *what) {
-        if (s == STY_OK) s = check_cuda(cudaMalloc(p, bytes), what);
+        if (s == STY_OK) s = check_cuda(device_malloc(p, bytes), what);
     };
     alloc((void **)&nr->w, np * 4, "alloc parameters");
     alloc((void **)&nr->m, np * 4, "alloc adam m");

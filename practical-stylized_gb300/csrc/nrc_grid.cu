@@ -663,13 +663,13 @@ sty_status ensure_cap(GridModel *g, uint64_t B) {
     STY_ARG_CHECK(B < (1ull << 31), "batch of %llu rows too large", (unsigned long long)B);
     const size_t wide = (size_t)std::max({g->H, g->E, kOpad});
     const size_t parts = tc_dw_partials_floats((int)B, std::max({g->H, g->E, kOpad}));
-    STY_TRY(check_cuda(cudaMalloc(&g->enc, B * g->E * 2), "alloc encoding"));
-    STY_TRY(check_cuda(cudaMalloc(&g->acts, (size_t)g->L * B * g->H * 2), "alloc activations"));
-    STY_TRY(check_cuda(cudaMalloc(&g->dp, B * wide * 2), "alloc layer gradient"));
-    STY_TRY(check_cuda(cudaMalloc(&g->dp2, B * wide * 2), "alloc layer gradient"));
-    STY_TRY(check_cuda(cudaMalloc(&g->z, B * wide * 4), "alloc output"));
-    STY_TRY(check_cuda(cudaMalloc(&g->dh, B * wide * 4), "alloc encoding gradient"));
-    STY_TRY(check_cuda(cudaMalloc(&g->parts, parts * 4), "alloc weight-gradient partials"));
+    STY_TRY(check_cuda(device_malloc(&g->enc, B * g->E * 2), "alloc encoding"));
+    STY_TRY(check_cuda(device_malloc(&g->acts, (size_t)g->L * B * g->H * 2), "alloc activations"));
+    STY_TRY(check_cuda(device_malloc(&g->dp, B * wide * 2), "alloc layer gradient"));
+    STY_TRY(check_cuda(device_malloc(&g->dp2, B * wide * 2), "alloc layer gradient"));
+    STY_TRY(check_cuda(device_malloc(&g->z, B * wide * 4), "alloc output"));
+    STY_TRY(check_cuda(device_malloc(&g->dh, B * wide * 4), "alloc encoding gradient"));
+    STY_TRY(check_cuda(device_malloc(&g->parts, parts * 4), "alloc weight-gradient partials"));
     g->cap = B;
     return STY_OK;
 }
@@ -712,7 +712,7 @@ sty_status grid_tc_forward(GridModel *g, bool ema, uint64_t count, const float *
         if (g->tiles) cudaFree(g->tiles);
         g->tiles = nullptr;
         g->tiles_cap = 0;
-        STY_TRY(check_cuda(cudaMalloc(&g->tiles, need), "alloc tile images"));
+        STY_TRY(check_cuda(device_malloc(&g->tiles, need), "alloc tile images"));
         g->tiles_cap = need;
     }
     GridTcArgs a;
@@ -832,14 +832,14 @@ sty_status grid_create(const sty_nrc_grid_config *c, GridModel **out, size_t *n_
     // (BF16 only: FP16 networks infer layer by layer on the same tensor-core GEMMs as training)
     g->tc = !g->f16 && (g->H == 32 || g->H == 64 || g->H == 128) && g->E <= kMaxE &&
             g->tc_smem + 64 <= (size_t)smem_optin;
-    sty_status s = check_cuda(cudaMalloc(&g->wb, (g->out_off + (size_t)kOpad * g->H) * 2), "alloc 16-bit weights");
-    if (s == STY_OK) s = check_cuda(cudaMalloc(&g->wb_ema, (g->out_off + (size_t)kOpad * g->H) * 2), "alloc 16-bit ema");
-    if (s == STY_OK) s = check_cuda(cudaMalloc(&g->tab16, g->n_tab * 2), "alloc fp16 tables");
-    if (s == STY_OK) s = check_cuda(cudaMalloc(&g->tab16_ema, g->n_tab * 2), "alloc fp16 ema tables");
-    if (s == STY_OK) s = check_cuda(cudaMalloc(&g->tsteps, g->n_tab * 4), "alloc table step counts");
+    sty_status s = check_cuda(device_malloc(&g->wb, (g->out_off + (size_t)kOpad * g->H) * 2), "alloc 16-bit weights");
+    if (s == STY_OK) s = check_cuda(device_malloc(&g->wb_ema, (g->out_off + (size_t)kOpad * g->H) * 2), "alloc 16-bit ema");
+    if (s == STY_OK) s = check_cuda(device_malloc(&g->tab16, g->n_tab * 2), "alloc fp16 tables");
+    if (s == STY_OK) s = check_cuda(device_malloc(&g->tab16_ema, g->n_tab * 2), "alloc fp16 ema tables");
+    if (s == STY_OK) s = check_cuda(device_malloc(&g->tsteps, g->n_tab * 4), "alloc table step counts");
     if (s == STY_OK) s = check_cuda(cudaMemset(g->tsteps, 0, g->n_tab * 4), "zero table step counts");
-    if (s == STY_OK && g->tc) s = check_cuda(cudaMalloc(&g->img, g->img_elems * 2), "alloc weight images");
-    if (s == STY_OK && g->tc) s = check_cuda(cudaMalloc(&g->img_ema, g->img_elems * 2), "alloc ema images");
+    if (s == STY_OK && g->tc) s = check_cuda(device_malloc(&g->img, g->img_elems * 2), "alloc weight images");
+    if (s == STY_OK && g->tc) s = check_cuda(device_malloc(&g->img_ema, g->img_elems * 2), "alloc ema images");
     if (s != STY_OK) {
         grid_destroy(g);
         return s;
@@ -864,9 +864,9 @@ sty_status grid_init_params(GridModel *g, uint64_t seed, float *w, cudaStream_t 
         fo.push_back(l == g->L ? g->O : g->H);
     }
     if (!g->d_fan_in) {
-        STY_TRY(check_cuda(cudaMalloc(&g->d_fan_in, fi.size() * sizeof(int)), "alloc fans"));
-        STY_TRY(check_cuda(cudaMalloc(&g->d_fan_out, fo.size() * sizeof(int)), "alloc fans"));
-        STY_TRY(check_cuda(cudaMalloc(&g->d_loff, g->loff.size() * sizeof(size_t)), "alloc offsets"));
+        STY_TRY(check_cuda(device_malloc(&g->d_fan_in, fi.size() * sizeof(int)), "alloc fans"));
+        STY_TRY(check_cuda(device_malloc(&g->d_fan_out, fo.size() * sizeof(int)), "alloc fans"));
+        STY_TRY(check_cuda(device_malloc(&g->d_loff, g->loff.size() * sizeof(size_t)), "alloc offsets"));
     }
     STY_TRY(check_cuda(cudaMemcpyAsync(g->d_fan_in, fi.data(), fi.size() * sizeof(int), cudaMemcpyHostToDevice, st),
                        "upload fans"));

@@ -464,11 +464,11 @@ extern "C" sty_status sty_pf_adjoint(const sty_pf_records *rec, uint32_t depth, 
     const int gx = (Wd + TW - 1) / TW, gy = (Hd + TH - 1) / TH, nb = gx * gy;
     const int npix = Wd * Hd, lb = (npix + 255) / 256;
     float *out = nullptr, *dimg = nullptr, *parts = nullptr, *lparts = nullptr, *lsum = nullptr;
-    sty_status s = check_cuda(cudaMallocAsync((void **)&out, 3 * N * 4, st), "alloc adjoint out");
-    if (s == STY_OK) s = check_cuda(cudaMallocAsync((void **)&dimg, (size_t)npix * 3 * 4, st), "alloc dimg");
-    if (s == STY_OK) s = check_cuda(cudaMallocAsync((void **)&parts, (size_t)nb * NG * 4, st), "alloc partials");
-    if (s == STY_OK) s = check_cuda(cudaMallocAsync((void **)&lparts, (size_t)lb * 4, st), "alloc loss partials");
-    if (s == STY_OK) s = check_cuda(cudaMallocAsync((void **)&lsum, 4, st), "alloc loss");
+    sty_status s = check_cuda(device_malloc_async((void **)&out, 3 * N * 4, st), "alloc adjoint out");
+    if (s == STY_OK) s = check_cuda(device_malloc_async((void **)&dimg, (size_t)npix * 3 * 4, st), "alloc dimg");
+    if (s == STY_OK) s = check_cuda(device_malloc_async((void **)&parts, (size_t)nb * NG * 4, st), "alloc partials");
+    if (s == STY_OK) s = check_cuda(device_malloc_async((void **)&lparts, (size_t)lb * 4, st), "alloc loss partials");
+    if (s == STY_OK) s = check_cuda(device_malloc_async((void **)&lsum, 4, st), "alloc loss");
     if (s == STY_OK)
         s = run_adjoint(rec, depth, radius, prm, n_steps, in_next, target, out, dimg, parts, lparts, lsum, grad, st);
     if (s == STY_OK && loss_out) {

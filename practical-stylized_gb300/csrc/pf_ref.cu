@@ -758,7 +758,7 @@ sty_status sty_pf_ref_create(uint64_t max_vertices, uint32_t table_size, sty_pf_
     const size_t n = max_vertices;
     sty_status st = STY_OK;
     auto alloc = [&](void **p, size_t bytes, const char *what) {
-        if (st == STY_OK) st = check_cuda(cudaMalloc(p, bytes), what);
+        if (st == STY_OK) st = check_cuda(device_malloc(p, bytes), what);
     };
     alloc((void **)&c->act, n * 4, "alloc act");
     alloc((void **)&c->num, 4, "alloc num");

@@ -27,10 +27,35 @@ struct sty_scene {
     float *light_cdf = nullptr;
     void *render_cache = nullptr;  // device buffers of the last render, reused by the next (trace.cu)
     // one parked device workspace, taken by a call that is given it and handed back when its work is done
-    std::mutex workspace_lock;
     void *workspace = nullptr;
     size_t workspace_bytes = 0;
+    sty_scene *next_parked = nullptr;
 };
+
+namespace {
+// every scene's parked workspace is under this lock; the list of the scenes that have one
+std::mutex g_parked_lock;
+sty_scene *g_parked = nullptr;
+// the scene's workspace, which is no longer parked (lock held)
+void *unpark(sty_scene *s, size_t *bytes) {
+    void *p = s->workspace;
+    *bytes = s->workspace_bytes;
+    s->workspace = nullptr;
+    s->workspace_bytes = 0;
+    for (sty_scene **q = &g_parked; *q; q = &(*q)->next_parked)
+        if (*q == s) {
+            *q = s->next_parked;
+            break;
+        }
+    s->next_parked = nullptr;
+    return p;
+}
+void drop_workspace(sty_scene *s) {
+    std::lock_guard<std::mutex> g(g_parked_lock);
+    size_t bytes = 0;
+    if (void *p = unpark(s, &bytes)) cudaFree(p);
+}
+}  // namespace
 
 namespace sty {
 SceneView scene_view(const sty_scene *s) {
@@ -58,7 +83,7 @@ namespace {
 
 void free_scene(sty_scene *s) {
     render_cache_free(s->render_cache);
-    if (s->workspace) cudaFree(s->workspace);
+    drop_workspace(s);
     void *ptrs[] = {s->nodes, s->tris, s->tri_material, s->tri_normal, s->tri_area,
                     s->tri_pos, s->materials, s->light_tris, s->light_cdf};
     for (void *p : ptrs)
@@ -159,7 +184,7 @@ sty_status sty_scene_create(const float *pos, const uint32_t *tmat, uint32_t n, 
     sty_status st = STY_OK;
     auto up = [&](void **dst, const void *src, size_t bytes, const char *what) {
         if (st != STY_OK || bytes == 0) return;
-        st = check_cuda(cudaMalloc(dst, bytes), what);
+        st = check_cuda(device_malloc(dst, bytes), what);
         if (st == STY_OK) st = check_cuda(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice), what);
     };
     int stack = 0, width = 0;
@@ -187,6 +212,15 @@ sty_status sty_scene_destroy(sty_scene *s) {
     return STY_OK;
 }
 
+sty_status sty_scene_trim(sty_scene *s) {
+    clear_error();
+    STY_ARG_CHECK(s, "sty_scene_trim: null scene");
+    drop_workspace(s);
+    render_cache_free(s->render_cache);
+    s->render_cache = nullptr;
+    return STY_OK;
+}
+
 sty_status sty_scene_closest_hit(sty_scene *s, const float *rays, uint64_t n, uint32_t *prim, float *t, float *bary,
                                  void *stream) {
     clear_error();
@@ -201,20 +235,19 @@ sty_status sty_scene_closest_hit(sty_scene *s, const float *rays, uint64_t n, ui
 // accessors used by the render driver
 namespace sty {
 const sty_camera &scene_camera(const sty_scene *s) { return s->camera; }
-sty_status scene_take_workspace(sty_scene *s, size_t bytes, void **ptr, size_t *got) {
+sty_status scene_take_workspace(sty_scene *s, size_t bytes, size_t most, void **ptr, size_t *got) {
     void *p = nullptr;
     size_t have = 0;
     {
-        std::lock_guard<std::mutex> g(s->workspace_lock);
-        std::swap(p, s->workspace);
-        std::swap(have, s->workspace_bytes);
+        std::lock_guard<std::mutex> g(g_parked_lock);
+        p = unpark(s, &have);
     }
-    if (p && have < bytes) {
+    if (p && (have < bytes || have > std::max(bytes, most))) {
         cudaFree(p);
         p = nullptr;
     }
     if (!p) {
-        STY_TRY(check_cuda(cudaMalloc(&p, bytes), "alloc scene workspace"));
+        STY_TRY(check_cuda(device_malloc(&p, bytes), "alloc scene workspace"));
         have = bytes;
     }
     *ptr = p;
@@ -224,14 +257,25 @@ sty_status scene_take_workspace(sty_scene *s, size_t bytes, void **ptr, size_t *
 void scene_give_workspace(sty_scene *s, void *p, size_t bytes) {
     constexpr size_t kKeep = (size_t)8 << 30;
     if (bytes <= kKeep) {
-        std::lock_guard<std::mutex> g(s->workspace_lock);
+        std::lock_guard<std::mutex> g(g_parked_lock);
         if (!s->workspace) {
             s->workspace = p;
             s->workspace_bytes = bytes;
+            s->next_parked = g_parked;
+            g_parked = s;
             return;
         }
     }
     cudaFree(p);
+}
+bool release_workspaces() {
+    std::lock_guard<std::mutex> g(g_parked_lock);
+    const bool any = g_parked != nullptr;
+    while (g_parked) {
+        size_t bytes = 0;
+        cudaFree(unpark(g_parked, &bytes));
+    }
+    return any;
 }
 void *&scene_render_cache(sty_scene *s) { return s->render_cache; }
 void scene_bounds(const sty_scene *s, float mn[3], float mx[3]) {

@@ -304,10 +304,11 @@ __device__ inline bool trace_any(const SceneView &s, const float o[3], const flo
 }
 
 SceneView scene_view(const sty_scene *s);
-// A device workspace of at least `bytes`: the one the scene has parked, or a new one. It belongs to the call until
-// it gives it back, which it does when no work on it is in flight. A scene keeps one of at most 8 GB until it is
-// destroyed; others are freed. Safe from several threads.
-sty_status scene_take_workspace(sty_scene *s, size_t bytes, void **ptr, size_t *got);
+// A device workspace of at least `bytes`: the one the scene has parked, unless that is larger than `most` (and than
+// `bytes`), or a new one. It belongs to the call until it gives it back, which it does when no work on it is in flight. A scene
+// keeps one of at most 8 GB until it is trimmed or destroyed, or until an allocation of this library finds memory short
+// (release_workspaces); others are freed. Safe from several threads.
+sty_status scene_take_workspace(sty_scene *s, size_t bytes, size_t most, void **ptr, size_t *got);
 void scene_give_workspace(sty_scene *s, void *ptr, size_t bytes);
 // device buffers kept by a scene between renders (defined in trace.cu)
 void render_cache_free(void *cache);

@@ -810,7 +810,7 @@ struct TraceJob {
             if (cache->p[k]) cudaFree(cache->p[k]);
             cache->p[k] = nullptr;
             cache->bytes[k] = 0;
-            s = check_cuda(cudaMalloc(&cache->p[k], bytes), what);
+            s = check_cuda(device_malloc(&cache->p[k], bytes), what);
             if (s != STY_OK) return nullptr;
             cache->bytes[k] = bytes;
         }

@@ -413,6 +413,10 @@ class Scene:
         except Exception:
             pass
 
+    def trim(self):
+        """Give back the device memory kept between calls (sty_scene_trim)."""
+        check(lib().sty_scene_trim(self.h))
+
     def closest_hit(self, rays):
         """rays: device float32 [n, 8] (o, d, tmin, tmax) -> (prim, t, bary) device tensors."""
         import torch
