@@ -529,7 +529,8 @@ __global__ void __launch_bounds__(256, 4) k_ref_filter(VArgs v, Geo g, const uin
         cnt += nb;
         queued -= nb;
     };
-    for (int cell = 0; cell < 27; cell++) {
+    for (unsigned cells = __ballot_sync(0xffffffffu, my_rg.x < my_rg.y); cells; cells &= cells - 1u) {  // those with points
+        const int cell = __ffs((int)cells) - 1;
         const uint2 rg = make_uint2(__shfl_sync(0xffffffffu, my_rg.x, cell), __shfl_sync(0xffffffffu, my_rg.y, cell));
         // 128 candidates per step, 4 l .. 4 l + 3 by lane l
         for (uint32_t base = rg.x & ~3u; base < rg.y; base += 128) {
@@ -588,10 +589,12 @@ __global__ void __launch_bounds__(256, 4) k_ref_filter(VArgs v, Geo g, const uin
         if (t < k) {
             const uint32_t u = (uint32_t)keys[t];
             list[t] = u;
-            const uint32_t mu = min(v.material[u], n_mats - 1);
-            const NbFrame f = make_frame(mats[mu], mu, ld3(v.ns, u), ld3(v.ng, u), ld3(v.wo, u));
-            frames[t] = f;
-            fl = (f.bits & 8u) != 0u;
+            if (prm.smis) {  // (only the pdf sums read them)
+                const uint32_t mu = min(v.material[u], n_mats - 1);
+                const NbFrame f = make_frame(mats[mu], mu, ld3(v.ns, u), ld3(v.ng, u), ld3(v.wo, u));
+                frames[t] = f;
+                fl = (f.bits & 8u) != 0u;
+            }
         }
         const unsigned bal = __ballot_sync(0xffffffffu, fl);
         if (lane == (int)r) flat = bal;
