@@ -520,8 +520,9 @@ __global__ void __launch_bounds__(256, 4) k_ref_filter(VArgs v, Geo g, const uin
         if (have && c < R) keys[c] = ((unsigned long long)c << 32) | sorted[kk];
         __syncwarp();
         if (have && c >= R) {
-            // (cells that share a bucket list its points once each: c can pass the number of points, and the table)
-            const uint32_t x = pcg_output(s_next), j = c < nact ? draw_below(x, c + 1u, so.magic[c]) : x % (c + 1u);
+            // (cells that share a bucket list its points once each: c can pass the number of points, and the table; asked
+            // for the whole warp)
+            const uint32_t x = pcg_output(s_next), j = cnt + 32u <= nact ? draw_below(x, c + 1u, so.magic[c]) : x % (c + 1u);
             if (j < R) atomicMax(&keys[j], ((unsigned long long)c << 32) | sorted[kk]);
             s_last = s_next;
             s_next = a32 * s_next + inc32;

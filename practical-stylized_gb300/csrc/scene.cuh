@@ -140,9 +140,10 @@ __device__ __forceinline__ RayBox ray_box(const float o[3], const float d[3]) {
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         r.o[a] = o[a];
-        const float v = fabsf(d[a]) < least ? copysignf(least, d[a]) : d[a];
-        // (an approximate reciprocal: its error scales both planes alike, far below the widening; it is 0 past 2^126)
-        r.inv[a] = fabsf(v) > 0x1p125f ? 1.0f / v : __fdividef(1.0f, v);
+        const float v = copysignf(fmaxf(fabsf(d[a]), least), d[a]);
+        // the approximate reciprocal of the whole range, subnormal results among it (__fdividef gives 0 past 2^126); its
+        // error scales both planes alike, far below the widening
+        asm("rcp.approx.f32 %0, %1;" : "=f"(r.inv[a]) : "f"(v));
     }
     return r;
 }
