@@ -482,7 +482,7 @@ def c3_bench(sty, reps: int = 20):
     depth-0 records with the filtered depth-1 result (radius 8, sigma_pos 0.05, sigma_nrm 0.2, toon
     0.1 / 0.3 / 0.6) as child input, radius 8, bandwidths (4, 0.05, 0.2). The loss target is the
     image the forward renders from the parameters perturbed by N(0, 0.05^2) (relative, seed 1). One
-    gradient = forward + loss + backward (weights recomputed, two sweeps), timed with CUDA events
+    gradient = forward + loss + backward (weights recomputed), timed with CUDA events
     over `reps` gradients; correctness against FP64 central differences is in the tests."""
     import ctypes as C
     import torch

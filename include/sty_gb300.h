@@ -329,7 +329,7 @@ STY_API sty_status sty_pf_ref_filter(sty_pf_ref_ctx *ctx, const sty_pf_vertices 
  * Parameters (36 floats, this order): [0] sharpness s, [1..8] thresholds t_k, [9..32] colours
  * c_k (rgb), [33] sigma_pixel, [34] sigma_pos, [35] sigma_nrm. `n_steps` (1..8) ramp steps are used;
  * gradients of unused thresholds / colours are 0. The backward recomputes the neighbourhood
- * weights (two sweeps per query) instead of storing them.
+ * weights instead of storing them.
  * `target` (device, width*height*3 floats, interleaved rgb); `grad` (device, 36 floats);
  * `loss_out` (host, optional; synchronises). `in_next` as in sty_pf_screen_filter_depth.
  * -------------------------------------------------------------------------------------- */

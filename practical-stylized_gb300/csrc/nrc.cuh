@@ -135,7 +135,8 @@ __device__ __forceinline__ void nrc_store_bf16(uint16_t *img, size_t i, float v)
 // truncates its accumulations, which takes ~0.7 x 2^-24 off a layer's outputs on average, and the
 // third piece, whose last place is 2^-25 of w, gives it back:
 // without it the outputs of a 5 x 64 network were 2.0e-7 too small on average, with it 1e-8 too large,
-// and |mean| <= 3e-8 over 1 to 8 layers.
+// and |mean| <= 3e-8 over 1 to 8 layers (a property of this chip's accumulators, not of the network: tests hold it to
+// 1e-7 at other weights).
 constexpr float kNrcUnbias = 4.2e-8f;
 size_t nrc_f32tc_image_elems(const NrcNet &n);
 // piece images of hidden weight i (flat parameter index, < layers * 64 * 64) for the value v

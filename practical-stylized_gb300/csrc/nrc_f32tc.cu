@@ -5,13 +5,15 @@
 // product a.w is the six piece products down to 2^-24 of it: a1w1, a1w2, a2w1, a2w2, a1w3, a3w1, each
 // exact, summed by tcgen05.mma into FP32 accumulators in TMEM. An accumulation truncates, so what
 // counts is how often a sum is cut at the result's magnitude: the small products go first, and
-// the four K steps of a1w1 are shared between the two accumulators, two cuts each (relative error
-// against FP64 of the 5 x 64 network 3.5e-7 with all four in one accumulator, 3.1e-7 so, 2.4e-7 with
-// the bias of the cuts given back, nrc.cuh; 4.1e-7 with FMA chains on the CUDA cores).
+// the four K steps of a1w1 are shared between the two accumulators, two cuts each (error of the outputs in the
+// 2-norm, relative, against FP64 for one 5 x 64 network: 3.5e-7 with all four in one accumulator, 3.1e-7 so, 2.4e-7
+// with the bias of the cuts given back, nrc.cuh; 4.1e-7 with FMA chains on the CUDA cores. Other weights and
+// inputs give other figures at about the same ratio: half to two thirds).
 //
-// Bound: the epilogues' instructions (load, ReLU, split, store of every activation): with 4 of the 18 MMAs
-// of a layer the kernel takes 95 % of its time. 2 073 600 queries 0.33 ms, 129 601 queries 29 us (the
-// register-tiled CUDA-core kernel this replaces: 1.99 ms, 164 us).
+// Bound: the chain of MMAs and epilogues (load, ReLU, split, store of every activation) of the two tiles an SM has room
+// for: the tensor pipe is busy 65 % of the time, issue slots 54 %; with 4 of the 18 MMAs of a layer the kernel takes 95 %
+// of its time. 2 073 600 queries 0.34 ms, 129 601 queries 30 us (the register-tiled CUDA-core kernel this replaces:
+// 1.99 ms, 164 us).
 //
 // Inference only: the training step stays on the CUDA cores (nrc.cu). Adam divides by the root of the
 // squared gradient, so weights whose gradient is all rounding follow that rounding; a training run

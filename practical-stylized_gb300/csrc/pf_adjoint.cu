@@ -144,11 +144,10 @@ __device__ __forceinline__ void row_any(const float *__restrict__ rowp, int plan
     }
 }
 
-// Bound by the FMA pipe and shared-memory reads (19 FFMA2 = 9.5 and 10 reads of 16 bytes = 10 SM cycles per 64 pairs
-// of a warp's 4 queries), with 12 warps per SM. 512 x 512, 4 spp, radius 8: the whole adjoint 3.06 ms with two
-// sweeps (the first for f and D), a candidate duplicated into each pair, 220 registers and one block of
-// 8 warps per SM; 1.88 with one sweep on the forward filter's f, 1.66 with blocks of 32 x 4 pixels, three
-// to an SM (32 x 12, one to an SM: 1.81).
+// Bound by the FMA pipe (60 % busy; the data pipe of L1 and shared memory 32 %) with 12 warps per SM, which do not cover
+// the staging of the rows and its barriers. 512 x 512, 4 spp, radius 8: the whole adjoint 3.06 ms with two sweeps (the
+// first for f and D), a candidate duplicated into each pair, 220 registers and one block of 8 warps per SM; 1.88 with one
+// sweep on the forward filter's f, 1.65 with blocks of 32 x 4 pixels, three to an SM (32 x 12, one to an SM: 1.81).
 template <int S, bool FIRST>
 __global__ void __launch_bounds__(NT, S == 4 ? 3 : 1) k_pf_adjoint(const AdjArgs a) {
     extern __shared__ __align__(16) float sm[];

@@ -139,7 +139,7 @@ struct Smem {
 // as the pairs (0, 1) and (2, 3) of the quad; part2[q][k].x / .y collect the even / odd samples of
 // query q (w, w*in).
 // Two quads per turn of the loop, so that the second's loads are in flight under the first's chains: 1080p, 4 spp,
-// 5 depths, radius 16 69.0 -> 67.4 ms, 16 spp at 256 x 256, radius 8 14.6 -> 14.5. Three or more do not
+// 5 depths, radius 16 69.0 -> 67.4 ms; 16 spp within noise. Three or more do not
 // fit the 128 registers (71.0 ms). The same with scalar FMAs: 76.4 ms.
 template <int S>
 __device__ __forceinline__ void row_pass_exp(const float *__restrict__ rowp, int plane, int qs, int lx, int R, float pix2,
