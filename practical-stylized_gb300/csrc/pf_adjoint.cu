@@ -381,7 +381,7 @@ sty_status sweep(const AdjArgs &a, int S, cudaStream_t st) {
 // largest): 1 sample 1.0, 2.8; 2 samples 1.6, 38 (2.8e-6 for 7e-8); 4 samples (whose filter subtracts a tile's
 // centre from the positions before it scales them) 0.9, 2.1; 8 samples 1.4, 12. The 2.1 and the like are surfaces with
 // sigma_nrm <= 0.05: the filter rounds the normal term's factor into the normals. The first sweep takes
-// 0.9 ms at 512 x 512, 4 spp, radius 8, where the whole is 1.65 without it.
+// 0.8 ms at 512 x 512, 4 spp, radius 8, where the whole is 1.65 without it (2 spp 0.91 and 0.65; before, with f always so, 1.08).
 bool sweep_gives_f(int spp, float sigma_nrm) { return spp == 2 || spp == 8 || sigma_nrm < 0.1f; }
 
 // everything both entry points launch, with their scratch: f 3 N floats, dimg 3 per pixel, parts NG per block, lparts one per
